@@ -96,6 +96,8 @@ struct Frame {
     DevBuf<uint32_t> order;  // tiles by decreasing range length: the raster CTAs' tile order
     DevBuf<uint32_t> order_hist;  // per-slice bin counts of the tile order (64 words per 1024 tiles)
     DevBuf<uint32_t> rgba8, n_contrib;
+    DevBuf<uint32_t> hit_masks;  // differentiable frames: the raster's hits per 8x4 block (RasterOut)
+    size_t mask_pitch = 0;
     DevBuf<float> rgb, final_t;
     DevBuf<float> grad2d, dl_stage;
     bool grad2d_zero = false;  // grad2d holds zeros (cleared by the last preprocess backward)
@@ -118,13 +120,13 @@ struct Frame {
         ctl.pads(l); view.pads(l); rec.pads(l); meta.pads(l); counts.pads(l); offsets.pads(l);
         for (int b = 0; b < 2; ++b) { keys[b].pads(l); vals[b].pads(l); }
         flags.pads(l); ranges.pads(l); order.pads(l); order_hist.pads(l); rgba8.pads(l); n_contrib.pads(l);
-        rgb.pads(l); final_t.pads(l); grad2d.pads(l); dl_stage.pads(l);
+        hit_masks.pads(l); rgb.pads(l); final_t.pads(l); grad2d.pads(l); dl_stage.pads(l);
     }
     void release() {
         ctl.release(); view.release(); rec.release(); meta.release(); counts.release(); offsets.release();
         for (int b = 0; b < 2; ++b) { keys[b].release(); vals[b].release(); }
         flags.release(); ranges.release(); rgba8.release(); n_contrib.release(); rgb.release(); final_t.release();
-        order.release(); order_hist.release(); grad2d.release(); dl_stage.release();
+        order.release(); order_hist.release(); hit_masks.release(); grad2d.release(); dl_stage.release();
         if (h_ctl) cudaFreeHost(h_ctl);
         h_ctl = nullptr;
     }
@@ -135,6 +137,7 @@ struct FrameArgs {
     const gs_scene* scene;
     const ViewBlock* view;  // device copy of the view block
     uint32_t n, w, h, tiles_x, tiles_y, passes, max_instance;
+    size_t mask_pitch;  // words per plane of the frame's hit masks
     RasterOut out;
 };
 
@@ -265,6 +268,7 @@ int frame_args(gs_ctx* ctx, const gs_scene* scene, const gs_view* view, FrameArg
     a->tiles_x = tiles_x;
     a->tiles_y = tiles_y;
     a->max_instance = scene->n * ctx->cfg.max_instance_factor;
+    a->mask_pitch = (size_t)a->max_instance / 32 + (size_t)tiles + 1;
     const uint32_t key_bits = 16u + bitlen((uint32_t)tiles - 1u);
     a->passes = (key_bits + ctx->cfg.digit_bits - 1) / ctx->cfg.digit_bits;
     return GS_OK;
@@ -275,7 +279,7 @@ int ensure_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a) {
     const uint32_t radix = 1u << ctx->cfg.digit_bits;
     const void* before[] = {f.rec.p, f.meta.p, f.counts.p, f.offsets.p, f.keys[0].p, f.keys[1].p, f.vals[0].p,
                             f.vals[1].p, f.flags.p, f.ranges.p, f.rgba8.p, f.rgb.p, f.final_t.p, f.n_contrib.p,
-                            f.order.p, f.order_hist.p};
+                            f.order.p, f.order_hist.p, f.hit_masks.p};
     GS_CK(f.rec.reserve((size_t)a.n * kRecFloat4));
     GS_CK(f.meta.reserve(a.n));
     GS_CK(f.counts.reserve(((size_t)a.n + 1 + 7) / 8 * 8));
@@ -299,9 +303,11 @@ int ensure_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a) {
     GS_CK(f.rgb.reserve(pix * 3));
     GS_CK(f.final_t.reserve(pix));
     GS_CK(f.n_contrib.reserve(pix));
+    if (ctx->cfg.flags & GS_FLAG_DIFFERENTIABLE)
+        GS_CK(f.hit_masks.reserve(a.mask_pitch * (ctx->cfg.tile_size * ctx->cfg.tile_size / 32)));
     const void* after[] = {f.rec.p, f.meta.p, f.counts.p, f.offsets.p, f.keys[0].p, f.keys[1].p, f.vals[0].p,
                            f.vals[1].p, f.flags.p, f.ranges.p, f.rgba8.p, f.rgb.p, f.final_t.p, f.n_contrib.p,
-                            f.order.p, f.order_hist.p};
+                           f.order.p, f.order_hist.p, f.hit_masks.p};
     if (std::memcmp(before, after, sizeof(before)) != 0) ++ctx->alloc_gen;
     return GS_OK;
 }
@@ -319,7 +325,7 @@ void* mapped_host(const void* p) {
     return attr.type == cudaMemoryTypeHost ? attr.devicePointer : nullptr;
 }
 
-RasterOut raster_out(const gs_ctx* ctx, Frame& f, const gs_image* out) {
+RasterOut raster_out(const gs_ctx* ctx, Frame& f, const gs_image* out, size_t mask_pitch) {
     const bool dev = out && out->location == GS_MEM_DEVICE;
     const bool keep = (ctx->cfg.flags & GS_FLAG_DIFFERENTIABLE) != 0;
     RasterOut ro{};
@@ -338,6 +344,8 @@ RasterOut raster_out(const gs_ctx* ctx, Frame& f, const gs_image* out) {
     if (keep) {
         ro.final_t = f.final_t.p;
         ro.n_contrib = f.n_contrib.p;
+        ro.hit_masks = f.hit_masks.p;
+        ro.mask_pitch = mask_pitch;
     } else if (out) {
         ro.final_t = out->final_t ? (dev ? out->final_t : f.final_t.p) : nullptr;
         ro.n_contrib = out->n_contrib ? (dev ? out->n_contrib : f.n_contrib.p) : nullptr;
@@ -393,6 +401,7 @@ void remember(Frame& f, const FrameArgs& a) {
     f.tiles_y = a.tiles_y;
     f.passes = a.passes;
     f.max_instance = a.max_instance;
+    f.mask_pitch = a.mask_pitch;
     f.sorted_buf = (int)(a.passes & 1u);
     f.valid = true;
 }
@@ -707,7 +716,7 @@ int gs_forward(gs_ctx* ctx, const gs_scene* scene, const gs_view* view, const gs
     rc = ensure_frame(ctx, f, a);
     if (rc != GS_OK) return rc;
     a.view = f.view.p;
-    a.out = raster_out(ctx, f, out);
+    a.out = raster_out(ctx, f, out, a.mask_pitch);
     {
         const uint32_t slot = ctx->next_slot;
         ctx->next_slot = (slot + 1) % kViewSlots;
@@ -791,7 +800,7 @@ static int forward_batch(gs_ctx* ctx, const gs_batch_view* views, uint32_t count
     }
     for (uint32_t i = 0; i < count; ++i) {
         args[i].view = ctx->d_bviews.p + i;
-        args[i].out = raster_out(ctx, *frames[i], &views[i].out);
+        args[i].out = raster_out(ctx, *frames[i], &views[i].out, args[i].mask_pitch);
         k.ptrs.insert(k.ptrs.end(), {views[i].scene, args[i].out.rgba8, args[i].out.rgb, args[i].out.final_t,
                                      args[i].out.n_contrib});
         k.dims.insert(k.dims.end(), {args[i].n, args[i].w, args[i].h});
@@ -1004,8 +1013,8 @@ static int enqueue_raster_backward(gs_ctx* ctx, Frame& f, const gs_scene* scene,
     if (scene->n && !f.grad2d_zero) GS_CK(cudaMemsetAsync(f.grad2d.p, 0, f.grad2d.cap * sizeof(float), s));
     f.grad2d_zero = false;
     if (ev) cudaEventRecord(ev[0], s);
-    launch_raster_backward(ctx->cfg.tile_size, ctx->cfg.raster_batch, f.ranges.p, f.vals[f.sorted_buf].p, f.rec.p,
-                           scene->n, f.ctl.p, f.width, f.height, f.tiles_x, f.tiles_y, f.final_t.p, f.n_contrib.p, dl,
+    launch_raster_backward(ctx->cfg.tile_size, f.ranges.p, f.vals[f.sorted_buf].p, f.rec.p, scene->n, f.ctl.p, f.width,
+                           f.height, f.tiles_x, f.tiles_y, f.final_t.p, f.n_contrib.p, f.hit_masks.p, f.mask_pitch, dl,
                            f.grad2d.p, f.order.p, s);
     if (ev) cudaEventRecord(ev[1], s);
     GS_CK(cudaGetLastError());

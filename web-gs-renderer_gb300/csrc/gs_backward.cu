@@ -1,11 +1,11 @@
 // gs_backward.cu -- the raster half of the gradients of the splat pipeline (no counterpart in the
 // reference, which only renders):
-//   k_raster_backward     per tile, walks each pixel's blended splats back to front from its last
-//                         contributor, recomputing power and alpha bit for bit as the forward did
-//                         (same pinned arithmetic, the forward's warp cull octagon), recovering T by
-//                         division, and accumulating dL/d(pixel.xy, conic, opacity, colour) per
-//                         Gaussian: two pixels per lane, the warp reduces by shuffles, nine lanes
-//                         issue the atomics.
+//   k_raster_backward     per 8x4 pixel block, walks the splats that the forward's warp of the block
+//                         visited (its hit masks) back to front from the block's last contributor,
+//                         recomputing power and alpha bit for bit as the forward did (same pinned
+//                         arithmetic), recovering T by division, and accumulating dL/d(pixel.xy, conic,
+//                         opacity, colour) per Gaussian: eight hits at a time reduced over the block's
+//                         pixels by matrix instructions, three vector atomics per hit.
 // The preprocess half (2D gradients -> the 59 attributes) is in gs_preprocess_backward.cu.
 // Conventions: gradients flow through the fp32 RGB before quantization; culled Gaussians, skipped
 // pairs and splats after a pixel's termination get none; active clamps (alpha 0.99, colour >= 0)
@@ -17,44 +17,57 @@
 namespace gs {
 namespace {
 
-__device__ __forceinline__ float hw_exp2(float x) {
+// ---- reduction of a hit's gradients on the tensor cores --------------------------------------------
+// With P_k(u, v) = {1, u, v, u^2, uv, v^2} over the pixel's offset (u, v) from its block's centre and
+// gp = dL/dpower of a (pixel, splat) pair, w = alpha T its blending weight, the nine gradients of a splat
+// over a warp's pixels follow from nine sums: the six moments sum(gp P_k) (dx = X - u and dy = Y - v are
+// affine in the pixel, so the sums of gp dx^i dy^j are polynomials in the splat's X, Y with the moments as
+// coefficients; dL/do is the zeroth over o) and the three sum(w dC). That is a matrix product of the
+// hits' [gp; w] rows with fixed columns: a pixel adds two values per hit instead of accumulating nine,
+// and eight hits at a time are reduced by mma.sync m16n8k8 (tf32, fp32 accumulators): rows 0-7 the hits'
+// gp, rows 8-15 their w, k the warp's pixels, columns either P_k (small multiples of 1/4: exact in tf32)
+// or dC split into its tf32 head and tail. gp and w are split into head and tail too (an mma reads the
+// upper 19 bits of an operand), so a product keeps 22 bits and more, and the accumulators are fp32.
+constexpr uint32_t kHits = 8;  // hits per flush
+
+__device__ __forceinline__ void mma_tf32(float d[4], const float a[4], float b0, float b1, const float c[4]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
+          "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+
+// tf32 head of v, rounded to nearest (two integer operations; cvt.rna.tf32.f32 takes four here); v minus it
+// is exact and serves as the second operand, of which the mma drops at most the last bit.
+__device__ __forceinline__ float tf32_head(float v) {
+    return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u);
+}
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+
+// Predicated adds to global memory (no branch around them).
+__device__ __forceinline__ void red_add4_if(bool on, float* p, float x, float y, float z, float w) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n @q red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n}"
+                 ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w), "r"((uint32_t)on) : "memory");
+}
+__device__ __forceinline__ void red_add_if(bool on, float* p, float x) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q red.global.add.f32 [%0], %1;\n}"
+                 ::"l"(p), "f"(x), "r"((uint32_t)on) : "memory");
+}
+
+// 1 / x for a normal x (a single instruction: no denormals, so no range handling; 1 ulp).
+__device__ __forceinline__ float fast_rcp(float x) {
     float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// Warp reduce-scatter of eight values: after it, each lane holds the warp total of value
-// (lane >> 2) & 7. Halving stages: xor 16 splits the values 0-3 | 4-7 between the half-warps, xor 8
-// splits each half again, xor 4 once more (4 + 2 + 1 shuffles), then xor 2 and xor 1 finish the
-// sums: 9 shuffles instead of 40 for eight separate reductions.
-__device__ __forceinline__ float warp_reduce_scatter8(const float v[8]) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const bool b4 = lane & 16u, b3 = lane & 8u, b2 = lane & 4u;
-    float w[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float send = b4 ? v[k] : v[k + 4];
-        const float keep = b4 ? v[k + 4] : v[k];
-        w[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-    float u[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const float send = b3 ? w[k] : w[k + 2];
-        const float keep = b3 ? w[k + 2] : w[k];
-        u[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-    const float send = b2 ? u[0] : u[1];
-    float t = (b2 ? u[1] : u[0]) + __shfl_xor_sync(0xffffffffu, send, 4);
-    t += __shfl_xor_sync(0xffffffffu, t, 2);
-    t += __shfl_xor_sync(0xffffffffu, t, 1);
-    return t;
 }
 
 // One pixel's backward state: its last contributor L (1-based position in the tile range), the
@@ -86,228 +99,287 @@ __device__ __forceinline__ void pix_load(PixState& p, uint32_t x, uint32_t y, ui
 }
 
 // Visits the splat at 1-based range position pos for one pixel: the same power / exp / alpha
-// decisions as the forward (bit for bit), then adds this pixel's share of the splat's gradients to
-// g = {d px, d py, d conic.x, d conic.y, d conic.z, d opacity, d r, d g, d b}, the first five without
-// their constant factors (-1, -1, -1/2, -1, -1/2, applied after the warp reduction). T is recovered by
-// division (the approximate reciprocal, 2 ulp, of 1 - alpha >= 0.01 is accurate enough for a
-// gradient). With C = sum_i alpha_i T_i c_i and T_{i+1} = T_i (1 - alpha_i),
+// decisions as the forward (bit for bit); gp = dL/dpower and its blending weight w, zeros if the pixel
+// did not blend it. T is recovered by division (the approximate reciprocal, 1 ulp, of 1 - alpha >= 0.01 is
+// accurate enough for a gradient). With C = sum_i alpha_i T_i c_i and T_{i+1} = T_i (1 - alpha_i),
 // dC/dalpha_i = T_i c_i - S_i / (1 - alpha_i), S_i being the colour added behind splat i, so
 // dL/dalpha_i = T_i K_i - D_i / (1 - alpha_i) with K_i = dC . c_i and D_i = dC . S_i, and D grows by
-// alpha_i T_i K_i per step: one running sum per pixel instead of three (S_r, S_g, S_b), and six fewer
-// instructions per step.
-// FIRST: g is written rather than added to (zeros when the pixel does not contribute), so the hit's
-// accumulators need no zeroing before the lane's first pixel.
-template <bool FIRST>
-__device__ __forceinline__ bool pix_step(PixState& p, uint32_t pos, const float4& a, const float4& b,
-                                         const float2& c, float g[9]) {
-    auto none = [&]() {
-        if (FIRST)
-#pragma unroll
-            for (int k = 0; k < 9; ++k) g[k] = 0.0f;
-        return false;
-    };
-    auto acc = [&](int k, float x, float y) { g[k] = FIRST ? x * y : __fmaf_rn(x, y, g[k]); };
+// alpha_i T_i K_i per step. No branch on the rejections: a rejected pixel takes alpha = 0 and K = 0, which
+// leaves its state as it is and gives two zeros.
+__device__ __forceinline__ void pix_step(PixState& p, uint32_t pos, const float4& a, const float4& b,
+                                         const float2& c, float& gp, float& w) {
     const float dx = a.x - p.fx, dy = a.y - p.fy;
     const float power = __fmaf_rn(-0.5f, __fmaf_rn(a.z * dx, dx, (b.x * dy) * dy), -((a.w * dx) * dy));
-    if (pos > p.L || power > 0.0f || power < c.y) return none();
-    // The gradient's value only needs exp to a few ulp: 2^(power log2 e) by the hardware's base-2
-    // exponential (one multiply and one MUFU op; its relative error and that of the rounded argument
-    // stay under 5e-7 on the raster's range [-5.6, 0], where no result is denormal, so flushing to
-    // zero changes nothing). The decisions must be the forward's, bit for bit: alpha >= 1/255 and the
-    // 0.99 clamp are taken on o * exp(power), so where that product lies within 1e-5 (relative) of
-    // either threshold the pinned raster exp is evaluated and decides.
-    float G = hw_exp2(power * 1.44269504f);
-    float og = b.y * G;
-    if (fabsf(og - kEpsilon) <= 1e-5f * kEpsilon || fabsf(og - kAlphaClamp) <= 1e-5f * kAlphaClamp) {
-        G = raster_expf(power);
-        og = b.y * G;
-    }
-    const float alpha = fminf(kAlphaClamp, og);
-    if (!(alpha >= kEpsilon)) return none();
-    // from here on only gradients are formed: fused multiply-adds are fine (the decisions above
+    const float og = raster_alpha_unclamped(b.y, power);  // the forward's o * exp(power)
+    float alpha = fminf(kAlphaClamp, og);
+    // from here on only gradients are formed: fused multiply-adds are fine (the decisions
     // follow the forward's pinned arithmetic)
-    const float ria = __fdividef(1.0f, 1.0f - alpha);
-    const float Tb = p.T * ria;  // transmittance in front of this splat
-    const float w = alpha * Tb;
-    acc(6, w, p.dr);
-    acc(7, w, p.dg);
-    acc(8, w, p.db);
-    const float k = __fmaf_rn(b.z, p.dr, __fmaf_rn(b.w, p.dg, c.x * p.db));  // dC . c
-    const float dalpha = __fmaf_rn(Tb, k, -(p.d * ria));
-    {
-        // a clamped alpha passes no gradient to power and opacity (a select, not a branch: 0.585 ->
-        // 0.580 ms per 1M / 1080p backward); the constant factors of d power / d(px, py, conic)
-        // (-1, -1, -1/2, -1, -1/2) are applied once per splat after the warp reduction (kGradSign)
-        const float da = og <= kAlphaClamp ? dalpha : 0.0f;
-        const float gp = da * og;  // dL/dpower
-        const float gpdx = gp * dx, gpdy = gp * dy;
-        acc(0, gp, __fmaf_rn(a.z, dx, a.w * dy));
-        acc(1, gp, __fmaf_rn(b.x, dy, a.w * dx));
-        acc(2, gpdx, dx);
-        acc(3, gpdx, dy);
-        acc(4, gpdy, dy);
-        acc(5, da, G);
-    }
+    float k = __fmaf_rn(b.z, p.dr, __fmaf_rn(b.w, p.dg, c.x * p.db));  // dC . c
+    const bool in = (pos <= p.L) & !(power > 0.0f) & !(power < c.y) & (alpha >= kEpsilon);
+    alpha = in ? alpha : 0.0f;
+    k = in ? k : 0.0f;
+    const float ria = fast_rcp(1.0f - alpha);
+    p.T = p.T * ria;  // transmittance in front of this splat
+    w = alpha * p.T;
+    const float dalpha = __fmaf_rn(p.T, k, -(p.d * ria));
+    gp = og <= kAlphaClamp ? dalpha * alpha : 0.0f;  // a clamped alpha passes no gradient
     p.d = __fmaf_rn(w, k, p.d);
-    p.T = Tb;
-    return true;
 }
 
-// One CTA per tile with TILE*TILE/2 threads: each warp owns an 8x8 pixel block and each lane two
-// pixels of it, (x, y) and (x, y + 4), so the per-splat warp reduction and shared-memory loads are
-// shared by two pixels. A warp walks only positions up to the largest last-contributor index of its
-// own pixels.
-template <int TILE, int BATCH>
-__global__ void __launch_bounds__(TILE * TILE / 2) k_raster_backward(const uint32_t* __restrict__ ranges,
+__device__ __forceinline__ bool pix_finite(const PixState& p) {
+    return finite_f(p.dr) && finite_f(p.dg) && finite_f(p.db);
+}
+
+// A pixel whose dL/dC is not finite stays out of the matrix products (a zero weight times it would be
+// NaN in every hit of its warp): it walks its part of the tile's list by itself and adds its gradients
+// one by one.
+__device__ __noinline__ void walk_alone(PixState p, const uint32_t* __restrict__ vals, uint32_t len,
+                                        const float4* __restrict__ rec, uint32_t n, float* __restrict__ grad2d) {
+    for (uint32_t pos = min(p.L, len); pos > 0u; --pos) {
+        const uint32_t gi = vals[pos - 1u];
+        if (gi >= n) continue;
+        const float4 a = rec[(size_t)kRecFloat4 * gi], b = rec[(size_t)kRecFloat4 * gi + 1];
+        const float4 r2 = rec[(size_t)kRecFloat4 * gi + 2];
+        float gp, w;
+        pix_step(p, pos, a, b, make_float2(r2.x, r2.y), gp, w);
+        if (w == 0.0f) continue;  // not blended (a blended pair's weight is positive)
+        const float dx = a.x - p.fx, dy = a.y - p.fy;
+        float* q = grad2d + (size_t)8 * gi;
+        atomicAdd(q + 0, -gp * (a.z * dx + a.w * dy));
+        atomicAdd(q + 1, -gp * (b.x * dy + a.w * dx));
+        atomicAdd(q + 2, w * p.dr);
+        atomicAdd(q + 3, w * p.dg);
+        atomicAdd(q + 4, -0.5f * gp * dx * dx);
+        atomicAdd(q + 5, -gp * dx * dy);
+        atomicAdd(q + 6, -0.5f * gp * dy * dy);
+        atomicAdd(q + 7, w * p.db);
+        atomicAdd(grad2d + (size_t)8 * n + gi, gp / b.y);
+    }
+}
+
+constexpr uint32_t kRowUnits = 20;  // 16-byte units per row: 16 pixel pairs, padded so that the eight
+                                    // lanes that read two rows at once hit distinct banks
+constexpr uint32_t kRing = 64;      // staged hits per warp (a multiple of kHits, at least 32 + 31)
+constexpr uint32_t kBwdWarps = 2;   // warps per CTA; they share nothing
+
+// Shared memory of a warp: a ring of staged hits and the rows of kHits of them. A unit of a row holds two
+// neighbouring lanes' (gp, w): the mma's k and k + 4.
+struct BwdWarp {
+    float4 a[kRing];  // (x, y, conic.x, conic.y)
+    float4 b[kRing];  // (conic.z, opacity, r, g)
+    float4 c[kRing];  // (b, cut, range position, Gaussian)
+    float4 rows[kHits * kRowUnits];
+};
+
+// One warp per 8x4 block, one lane per pixel, no barrier between warps. The forward left one word per
+// block and 32 range positions with a bit for each splat that its cull let through (hit_masks): the warp
+// reads them from the group of its pixels' largest last contributor down, and only the records of those
+// splats are staged, 32 positions at a time, by asynchronous copies into the ring while the hits staged
+// before are processed, eight at a time and fully unrolled. Against a CTA per tile that staged whole
+// batches, computed the cull again and met at two barriers per batch, a hit's bookkeeping (finding the
+// next bit, addresses, the counter of the pending rows) is gone.
+//
+// Bound by instruction issue (77% of slots at 28 warps per SM) where the blocks fill the GPU, by the
+// longest list otherwise. Measured against the CTA per tile with shuffle reductions and two pixels per
+// lane, mixture scenes: 1M / 1080p 427M -> 276M warp instructions, 839k -> 603k cycles; 3M / 1080p
+// 879 -> 640 us; 500k / 720p (a list of 2300 splats) 358 -> 150 us; 20k / 397x301 92 -> 30 us. On the way,
+// 1M / 1080p: matrix sums but a CTA per tile, 8x8 blocks with two pixels per lane 1008k cycles, 8x4 blocks
+// 847k; 8x4 blocks by the hit masks 693k; the chain's divide as one reciprocal and no branch in a hit
+// 664k; columns without selects and predicated atomics 631k; heads by integer rounding 603k.
+template <int TILE>
+__global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backward(const uint32_t* __restrict__ ranges,
                                                                      const uint32_t* __restrict__ vals,
                                                                      const float4* __restrict__ rec, uint32_t n,
                                                                      const FrameCtl* __restrict__ ctl,
                                                                      uint32_t width, uint32_t height,
-                                                                     uint32_t tiles_x,
+                                                                     uint32_t tiles_x, uint32_t tiles,
                                                                      const float* __restrict__ final_t,
                                                                      const uint32_t* __restrict__ n_contrib,
+                                                                     const uint32_t* __restrict__ hit_masks,
+                                                                     size_t mask_pitch,
                                                                      const float* __restrict__ dl_drgb,
                                                                      float* __restrict__ grad2d,
                                                                      const uint32_t* __restrict__ order) {
     pdl_wait();
-    constexpr int WX = TILE / 8;
-    constexpr int kThreads = TILE * TILE / 2;
-    __shared__ float4 s_a[BATCH];
-    __shared__ float4 s_b[BATCH];
-    __shared__ float2 s_c[BATCH];
-    __shared__ float4 s_box[BATCH];
-    __shared__ float4 s_diag[BATCH];
-    __shared__ uint32_t s_g[BATCH];
-    __shared__ uint32_t s_maxl;
+    constexpr uint32_t WX = TILE / 8, kTileWarps = TILE * TILE / 32;
+    constexpr float kCx = 3.5f, kCy = 1.5f;  // centre of a warp's block
+    __shared__ BwdWarp s_warp[kBwdWarps];
+    BwdWarp& sh = s_warp[threadIdx.x >> 5];
 
-    const uint32_t tile = order ? order[blockIdx.x] : blockIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t wid = blockIdx.x * kBwdWarps + (threadIdx.x >> 5);
+    const uint32_t warp = wid % kTileWarps;
+    if (wid / kTileWarps >= tiles) return;
+    const uint32_t tile = order ? order[wid / kTileWarps] : wid / kTileWarps;
     const uint32_t tx = tile % tiles_x, ty = tile / tiles_x;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t bx0 = tx * TILE + 8u * (warp % WX), by0 = ty * TILE + 8u * (warp / WX);
-    const uint32_t x = bx0 + (lane & 7u), y = by0 + (lane >> 3);
+    const uint32_t bx0 = tx * TILE + 8u * (warp % WX), by0 = ty * TILE + 4u * (warp / WX);
     const uint2 range = reinterpret_cast<const uint2*>(ranges)[tile];
     const uint32_t end = ctl ? min(range.y, ctl->sorted_count) : range.y;
     const uint32_t start = range.x;
     const uint32_t len = end > start ? end - start : 0u;
-    const float rx0 = (float)bx0, rx1 = (float)(bx0 + 7u), ry0 = (float)by0, ry1 = (float)(by0 + 7u);
-    const float tx0 = (float)(tx * TILE), tx1 = (float)(tx * TILE + TILE - 1u);
-    const float ty0 = (float)(ty * TILE), ty1 = (float)(ty * TILE + TILE - 1u);
 
-    // factor of the value this lane ends up holding after warp_reduce_scatter8 (see pix_step)
-    const float kGradSign[8] = {-1.0f, -1.0f, -0.5f, -1.0f, -0.5f, 1.0f, 1.0f, 1.0f};
-    const float sign = kGradSign[(lane >> 2) & 7u];
-    PixState p0, p1;
-    pix_load(p0, x, y, width, height, final_t, n_contrib, dl_drgb);
-    pix_load(p1, x, y + 4u, width, height, final_t, n_contrib, dl_drgb);
-    const uint32_t wmax = min(__reduce_max_sync(0xffffffffu, max(p0.L, p1.L)), len);
-    if (threadIdx.x == 0) s_maxl = 0;
-    __syncthreads();
-    if (lane == 0 && wmax) atomicMax(&s_maxl, wmax);
-    __syncthreads();
-    const uint32_t maxl = s_maxl;
-
-    // positions are 1-based within the tile range; walk batches (lo, hi] from the top down
-    for (uint32_t hi = maxl; hi > 0;) {
-        const uint32_t lo = hi > (uint32_t)BATCH ? hi - BATCH : 0u;
-        const uint32_t cnt = hi - lo;
-        __syncthreads();
-        for (uint32_t j = threadIdx.x; j < cnt; j += kThreads) {
-            const uint32_t g = vals[start + lo + j];
-            if (g < n) {
-                const float4 r0 = __ldg(rec + (size_t)kRecFloat4 * g);
-                const float4 r1 = __ldg(rec + (size_t)kRecFloat4 * g + 1);
-                const float4 r2 = __ldg(rec + (size_t)kRecFloat4 * g + 2);
-                s_a[j] = r0;
-                s_b[j] = r1;
-                s_c[j] = make_float2(r2.x, r2.y);
-                s_box[j] = cull_box(r0.x, r0.y, r0.z, r0.w, r1.x, r2.y, tx0, tx1, ty0, ty1, s_diag[j]);
-                s_g[j] = g;
-            } else {
-                const float inf = __int_as_float(0x7f800000);
-                s_box[j] = make_float4(inf, -inf, inf, -inf);
-                s_diag[j] = s_box[j];
-                s_g[j] = 0xFFFFFFFFu;
-            }
-        }
-        __syncthreads();
-        if (lo < wmax) {
-            // groups of 32 from the warp's top position in this batch down, splats in a group from
-            // high to low
-            const int top = (int)min(cnt, wmax - lo) - 1;
-            for (int gtop = top; gtop >= 0; gtop -= 32) {
-                const int gbase = gtop - 31;
-                const int jj = gbase + (int)lane;
-                const bool hit = jj >= 0 && box_meets(s_box[jj], rx0, rx1, ry0, ry1) &&
-                                 box_meets(s_diag[jj], rx0 + ry0, rx1 + ry1, rx0 - ry1, rx1 - ry0);
-                uint32_t m = __ballot_sync(0xffffffffu, hit);
-                while (m) {
-                    const int bit = 31 - __clz(m);
-                    m &= ~(1u << bit);
-                    const int j = gbase + bit;
-                    const uint32_t pos = lo + (uint32_t)j + 1u;
-                    const float4 a = s_a[j];
-                    const float4 b = s_b[j];
-                    const float2 c = s_c[j];
-                    float g[9];
-                    const bool c0 = pix_step<true>(p0, pos, a, b, c, g);
-                    const bool c1 = pix_step<false>(p1, pos, a, b, c, g);
-                    const uint32_t who = __ballot_sync(0xffffffffu, c0 || c1);
-                    if (__popc(who) > 8) {
-                        const float mine = sign * warp_reduce_scatter8(g);  // total of value (lane >> 2) & 7
-                        const float blue = warp_sum(g[8]);
-                        const uint32_t gi = s_g[j];
-                        if (gi < n) {
-                            float* dst = grad2d + (size_t)9 * gi;
-                            if ((lane & 3u) == 0u) atomicAdd(dst + ((lane >> 2) & 7u), mine);
-                            if (lane == 2u) atomicAdd(dst + 8, blue);
-                        }
-                    } else if (who) {
-                        // up to eight contributing lanes: each adds its own nine values (nine atomic
-                        // instructions for the warp either way) instead of the warp's reduce-scatter.
-                        // Measured at 1M / 1080p: up to 4 lanes 0.554 ms, 8 (or 10) 0.545, 16 0.653 (the
-                        // per-lane atomics then load L2 more than the reduce-scatter costs); 0.556 without
-                        const uint32_t gi = s_g[j];
-                        if ((c0 || c1) && gi < n) {
-                            float* dst = grad2d + (size_t)9 * gi;
-#pragma unroll
-                            for (int k = 0; k < 8; ++k) atomicAdd(dst + k, kGradSign[k] * g[k]);
-                            atomicAdd(dst + 8, g[8]);
-                        }
-                    }
-                }
-            }
-        }
-        hi = lo;
+    PixState p;
+    pix_load(p, bx0 + (lane & 7u), by0 + (lane >> 3), width, height, final_t, n_contrib, dl_drgb);
+    if (!pix_finite(p)) {
+        walk_alone(p, vals + start, len, rec, n, grad2d);
+        p.L = 0;
+        p.dr = p.dg = p.db = 0.0f;
     }
+    const uint32_t wmax = min(__reduce_max_sync(0xffffffffu, p.L), len);
+    if (wmax == 0u) return;
+    // this lane's part of the columns: column fr at the pixels of lanes 2 m and 2 m + 1, m = 4 i + fc, for
+    // step i of the product (offsets u = 2 fc + h - 3.5 and v = i - 1.5); the colour columns are r, g, b
+    // heads, one unused, r, g, b tails, one unused
+    const uint32_t fr = lane >> 2, fc = lane & 3u;
+    float poly[4][2], colour[4][2];
+    {
+        // P_k as a product of two of 1, u, v: 11, u1, v1, uu, uv, vv
+        const float f0 = fr == 0u ? 1.0f : 0.0f, fu = fr == 1u || fr == 3u || fr == 4u ? 1.0f : 0.0f, fv = 1.0f - f0 - fu;
+        const float g0 = fr < 3u ? 1.0f : 0.0f, gu = fr == 3u ? 1.0f : 0.0f, gv = 1.0f - g0 - gu;
+        float* const plane = reinterpret_cast<float*>(sh.rows);
+        plane[lane] = p.dr;
+        plane[32u + lane] = p.dg;
+        plane[64u + lane] = p.db;
+        plane[96u + lane] = 0.0f;
+        __syncwarp();
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; ++i) {
+            const float v = (float)i - kCy;
+            const float2 d2 = reinterpret_cast<const float2*>(plane)[16u * (fr & 3u) + 4u * i + fc];
+            const float d[2] = {d2.x, d2.y};
+#pragma unroll
+            for (uint32_t h = 0; h < 2u; ++h) {
+                const float u = (float)(2u * fc + h) - kCx;
+                poly[i][h] = (f0 + fu * u + fv * v) * (g0 + gu * u + gv * v);  // exact
+                const float head = tf32_head(d[h]);
+                colour[i][h] = fr < 4u ? head : d[h] - head;
+            }
+        }
+        __syncwarp();
+    }
+    const float cx = (float)bx0 + kCx, cy = (float)by0 + kCy;
+
+    // visits the eight staged hits from ring slot h0 on and adds the gradients of the first cnt of them
+    auto visit = [&](uint32_t h0, uint32_t cnt) {
+#pragma unroll
+        for (uint32_t u = 0; u < kHits; ++u) {
+            const float4 c = sh.c[h0 + u];
+            float gp, w;
+            pix_step(p, __float_as_uint(c.z), sh.a[h0 + u], sh.b[h0 + u], make_float2(c.x, c.y), gp, w);
+            reinterpret_cast<float2*>(sh.rows)[2u * kRowUnits * u + lane] = make_float2(gp, w);
+        }
+        __syncwarp();
+        float m[4] = {0.0f, 0.0f, 0.0f, 0.0f}, q[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; ++i) {
+            const float4 v = sh.rows[fr * kRowUnits + 4u * i + fc];
+            const float head[4] = {tf32_head(v.x), tf32_head(v.y), tf32_head(v.z), tf32_head(v.w)};
+            const float tail[4] = {v.x - head[0], v.y - head[1], v.z - head[2], v.w - head[3]};
+            mma_tf32(m, head, poly[i][0], poly[i][1], m);
+            mma_tf32(q, head, colour[i][0], colour[i][1], q);
+            mma_tf32(m, tail, poly[i][0], poly[i][1], m);
+            mma_tf32(q, tail, colour[i][0], colour[i][1], q);
+        }
+        // m[0..1]: moments 2 fc, 2 fc + 1 of hit fr; q[2..3]: colour columns 2 fc, 2 fc + 1
+        const float s0 = __shfl_sync(0xffffffffu, m[0], 0, 4), su = __shfl_sync(0xffffffffu, m[1], 0, 4);
+        const float sv = __shfl_sync(0xffffffffu, m[0], 1, 4), suu = __shfl_sync(0xffffffffu, m[1], 1, 4);
+        const float suv = __shfl_sync(0xffffffffu, m[0], 2, 4), svv = __shfl_sync(0xffffffffu, m[1], 2, 4);
+        const float c0 = q[2] + __shfl_xor_sync(0xffffffffu, q[2], 2);  // r (fc 0), b (fc 1)
+        const float c1 = q[3] + __shfl_xor_sync(0xffffffffu, q[3], 2);  // g (fc 0)
+        const float4 a = sh.a[h0 + fr];
+        const float2 b = *reinterpret_cast<const float2*>(&sh.b[h0 + fr]);
+        const uint32_t gi = __float_as_uint(sh.c[h0 + fr].w);
+        const float X = a.x - cx, Y = a.y - cy;
+        const float sx = __fmaf_rn(X, s0, -su), sy = __fmaf_rn(Y, s0, -sv);  // sums of gp dx, gp dy
+        const float sxx = __fmaf_rn(X, sx - su, suu), syy = __fmaf_rn(Y, sy - sv, svv);
+        const float sxy = __fmaf_rn(Y, sx, __fmaf_rn(-X, sv, suv));
+        const bool first = fc == 0u, valid = fr < cnt && gi < n;
+        red_add4_if(valid && fc < 2u, grad2d + (size_t)8 * gi + 4u * fc, first ? -__fmaf_rn(a.z, sx, a.w * sy) : -0.5f * sxx,
+                    first ? -__fmaf_rn(b.x, sy, a.w * sx) : -sxy, first ? c0 : -0.5f * syy, first ? c1 : c0);
+        red_add_if(valid && fc == 2u && s0 != 0.0f, grad2d + (size_t)8 * n + gi, s0 * fast_rcp(b.y));
+        __syncwarp();
+    };
+
+    // the groups of 32 positions with hits, from the top down: masks are read 32 groups at a time, and the
+    // Gaussian indices of a group are loaded while the group before it is staged
+    const uint32_t* const masks = hit_masks + (size_t)warp * mask_pitch + hit_mask_base(start, tile);
+    int32_t group = (int32_t)((wmax - 1u) >> 5) + 1;  // the group staged last
+    uint32_t words = 0, left = 0;   // the lane's mask word of the current 32 groups; how many are unread
+    uint32_t m = 0, gnext = n;      // the next group's mask and this lane's Gaussian in it
+    auto next_group = [&]() {
+        m = 0;
+        while (m == 0u && group > 0) {
+            --group;
+            if (left == 0u) {
+                left = 32u;
+                const int32_t at = group - (int32_t)lane;
+                words = at >= 0 ? masks[at] : 0u;
+            }
+            m = __shfl_sync(0xffffffffu, words, 32u - left);
+            --left;
+            const uint32_t last = wmax - ((uint32_t)group << 5);  // positions of the group that are visited
+            if (last < 32u) m &= (1u << last) - 1u;
+        }
+        if (m >> lane & 1u) gnext = vals[start + ((uint32_t)group << 5) + lane];
+    };
+
+    uint32_t head = 0, ready = 0, tail = 0;  // hits visited, staged for certain, staged or on their way
+    next_group();
+    while (true) {
+        while (m != 0u && tail - head <= kRing - 32u) {
+            if (m >> lane & 1u) {
+                const uint32_t slot = (tail + __popc(m >> lane) - 1u) % kRing;  // back to front
+                const bool ok = gnext < n;
+                const uint32_t g = ok ? gnext : 0u;
+                cp_async16(&sh.a[slot], rec + (size_t)kRecFloat4 * g);
+                cp_async16(&sh.b[slot], rec + (size_t)kRecFloat4 * g + 1);
+                cp_async8(&sh.c[slot], rec + (size_t)kRecFloat4 * g + 2);
+                // an index out of range only comes from a timed-out sort: a position no pixel blends
+                const uint32_t pos = ok ? ((uint32_t)group << 5) + lane + 1u : 0xFFFFFFFFu;
+                reinterpret_cast<uint2*>(&sh.c[slot])[1] = make_uint2(pos, ok ? g : n);
+            }
+            tail += __popc(m);
+            next_group();
+        }
+        cp_async_commit();
+        if (m == 0u) break;
+        cp_async_wait<1>();
+        __syncwarp();
+        for (uint32_t k = 0; k < 2u && ready - head >= kHits; ++k, head += kHits) visit(head % kRing, kHits);
+        ready = tail;
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    for (; head < tail; head += kHits) visit(head % kRing, min(kHits, tail - head));
 }
 
-template <int TILE>
-void launch_bwd_tile(uint32_t batch, const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n,
-                     const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
-                     const float* final_t, const uint32_t* n_contrib, const float* dl, float* grad2d,
-                     const uint32_t* order, cudaStream_t s) {
-    const uint32_t grid = tiles_x * tiles_y;
-    constexpr int threads = TILE * TILE / 2;
-    switch (batch) {
-        case 32: launch_pdl(k_raster_backward<TILE, 32>, dim3(grid), dim3(threads), s, ranges, vals, rec, n, ctl, width, height, tiles_x, final_t, n_contrib, dl, grad2d, order); break;
-        case 64: launch_pdl(k_raster_backward<TILE, 64>, dim3(grid), dim3(threads), s, ranges, vals, rec, n, ctl, width, height, tiles_x, final_t, n_contrib, dl, grad2d, order); break;
-        case 128: launch_pdl(k_raster_backward<TILE, 128>, dim3(grid), dim3(threads), s, ranges, vals, rec, n, ctl, width, height, tiles_x, final_t, n_contrib, dl, grad2d, order); break;
-        default: launch_pdl(k_raster_backward<TILE, 256>, dim3(grid), dim3(threads), s, ranges, vals, rec, n, ctl, width, height, tiles_x, final_t, n_contrib, dl, grad2d, order); break;
-    }
+template <int TILE, typename... Args>
+void launch_bwd_tile(uint32_t tiles, cudaStream_t s, Args&&... args) {
+    const uint32_t warps = tiles * (TILE * TILE / 32);
+    launch_pdl(k_raster_backward<TILE>, dim3((warps + kBwdWarps - 1u) / kBwdWarps), dim3(kBwdWarps * 32), s,
+               std::forward<Args>(args)...);
 }
 
 }  // namespace
 
-void launch_raster_backward(uint32_t tile, uint32_t batch, const uint32_t* ranges, const uint32_t* vals,
-                            const float4* rec, uint32_t n, const FrameCtl* ctl, uint32_t width, uint32_t height,
-                            uint32_t tiles_x, uint32_t tiles_y, const float* final_t, const uint32_t* n_contrib,
-                            const float* dl_drgb, float* grad2d, const uint32_t* order, cudaStream_t s) {
-    if (tile == 8)
-        launch_bwd_tile<8>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, final_t, n_contrib, dl_drgb, grad2d, order, s);
-    else if (tile == 32)
-        launch_bwd_tile<32>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, final_t, n_contrib, dl_drgb, grad2d, order, s);
-    else
-        launch_bwd_tile<16>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, final_t, n_contrib, dl_drgb, grad2d, order, s);
+void configure_raster_backward() {
+    cudaFuncSetAttribute(k_raster_backward<8>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaFuncSetAttribute(k_raster_backward<16>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaFuncSetAttribute(k_raster_backward<32>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+
+void launch_raster_backward(uint32_t tile, const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n,
+                            const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
+                            const float* final_t, const uint32_t* n_contrib, const uint32_t* hit_masks,
+                            size_t mask_pitch, const float* dl_drgb, float* grad2d, const uint32_t* order,
+                            cudaStream_t s) {
+    auto launch = [&](auto bwd) {
+        bwd(tiles_x * tiles_y, s, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_x * tiles_y, final_t, n_contrib,
+            hit_masks, mask_pitch, dl_drgb, grad2d, order);
+    };
+    if (tile == 8) launch([](auto&&... a) { launch_bwd_tile<8>(a...); });
+    else if (tile == 32) launch([](auto&&... a) { launch_bwd_tile<32>(a...); });
+    else launch([](auto&&... a) { launch_bwd_tile<16>(a...); });
 }
 
 }  // namespace gs

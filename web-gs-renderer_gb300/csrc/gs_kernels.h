@@ -24,18 +24,22 @@ void launch_pack_to_rows(const float* packed, uint32_t n, uint32_t stride, float
 // whole grid has drained (inside a captured graph the edge stays programmatic). k must call pdl_wait()
 // before anything else.
 template <typename... Params, typename... Args>
-inline void launch_pdl(void (*k)(Params...), dim3 grid, dim3 block, cudaStream_t s, Args&&... args) {
+inline void launch_pdl_smem(void (*k)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+}
+template <typename... Params, typename... Args>
+inline void launch_pdl(void (*k)(Params...), dim3 grid, dim3 block, cudaStream_t s, Args&&... args) {
+    launch_pdl_smem(k, grid, block, 0, s, std::forward<Args>(args)...);
 }
 
 // ---- frame ----------------------------------------------------------------------------------
@@ -140,7 +144,15 @@ struct RasterOut {
     float* rgb;          // W*H*3 or null
     float* final_t;      // W*H or null
     uint32_t* n_contrib; // W*H or null
+    uint32_t* hit_masks; // differentiable frames, or null: the splats that each warp's cull let through, one
+                         // word per 8x4 block and 32 range positions: word hit_mask_base(start, tile) + group
+                         // of plane `warp of the tile` (planes mask_pitch words apart); groups past the
+                         // block's termination are left unwritten. Only with n_contrib.
+    size_t mask_pitch;
 };
+// First word of a tile's groups in a plane: the tiles' starts grow with their index, so (start / 32 + tile)
+// leaves every tile ceil(length / 32) words of its own; a plane holds max_instance / 32 + tiles + 1.
+__host__ __device__ __forceinline__ size_t hit_mask_base(uint32_t start, uint32_t tile) { return (size_t)(start >> 5) + tile; }
 // ctl (optional) bounds every range by the sorted count; n bounds the Gaussian indices; order
 // (optional) is the tile each CTA renders (launch_tile_order), else CTA i renders tile i.
 void launch_raster(uint32_t tile, uint32_t batch, const uint32_t* ranges, const uint32_t* vals, const float4* rec,
@@ -163,12 +175,16 @@ void launch_camera_views(const gs_camera* cams, uint32_t n, ViewBlock* out, cuda
 cudaError_t static_scan_set_sequence(uint32_t seq);
 
 // ---- backward ---------------------------------------------------------------------------------
-// grad2d: 9 floats per Gaussian, dL/d(pixel.x, pixel.y, conic.x, conic.y, conic.z, opacity, r, g, b),
-// accumulated with atomics (zero it first).
-void launch_raster_backward(uint32_t tile, uint32_t batch, const uint32_t* ranges, const uint32_t* vals,
-                            const float4* rec, uint32_t n, const FrameCtl* ctl, uint32_t width, uint32_t height,
-                            uint32_t tiles_x, uint32_t tiles_y, const float* final_t, const uint32_t* n_contrib,
-                            const float* dl_drgb, float* grad2d, const uint32_t* order, cudaStream_t s);
+// grad2d: 9 floats per Gaussian, accumulated with atomics (zero it first): eight in one 32-byte row,
+// dL/d(pixel.x, pixel.y, r, g | conic.x, conic.y, conic.z, b), for two 16-byte vector atomics, then, from
+// float 8n on, dL/d(opacity). configure_raster_backward: kernel attributes, once per device.
+void configure_raster_backward();
+// hit_masks, mask_pitch: as the frame's forward raster left them (RasterOut).
+void launch_raster_backward(uint32_t tile, const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n,
+                            const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
+                            const float* final_t, const uint32_t* n_contrib, const uint32_t* hit_masks,
+                            size_t mask_pitch, const float* dl_drgb, float* grad2d, const uint32_t* order,
+                            cudaStream_t s);
 // Up to kMaxMultiViews views of one scene for launch_preprocess_backward_multi.
 struct MultiViewGrads {
     const ViewBlock* view[kMaxMultiViews];

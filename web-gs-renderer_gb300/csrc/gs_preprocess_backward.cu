@@ -16,13 +16,16 @@ constexpr uint32_t kBwdGroup = 128;  // Gaussians (threads) per preprocess-backw
 // packed write-out reads them with at most 4-way bank conflicts.
 constexpr uint32_t kBwdPitch = 132;
 
-// Chain rule of one visible Gaussian from its 2D gradients d2 = dL/d(pixel.xy, conic, opacity, rgb)
-// back to its 59 attributes. R_(row) reads an attribute, W_(row, v) emits its gradient; every W_ of a
+// Where grad2d keeps dL/d(pixel.x, pixel.y, conic.x, conic.y, conic.z, opacity, r, g, b): its place in the
+// Gaussian's row of eight, or 8 for the opacity, which has a plane of its own.
+__device__ constexpr int kGradPlace[9] = {0, 1, 4, 5, 6, 8, 2, 3, 7};
+
+// Chain rule of one visible Gaussian from its 2D gradients (D_(k): the k-th of dL/d(pixel.xy, conic,
+// opacity, rgb)) back to its 59 attributes. R_(row) reads an attribute, W_(row, v) emits its gradient; every W_ of a
 // row comes after the last R_ of that row, so W_ may overwrite the staged attribute in place.
-template <class RF, class WF, class SF>
-__device__ __forceinline__ void backward_gaussian(const ViewBlock& sv, const float* __restrict__ d2, RF R_, WF W_,
-                                                  SF sh_ready) {
-    const float gpx = d2[0], gpy = d2[1], gA = d2[2], gB = d2[3], gC = d2[4], go = d2[5];
+template <class DF, class RF, class WF, class SF>
+__device__ __forceinline__ void backward_gaussian(const ViewBlock& sv, DF D_, RF R_, WF W_, SF sh_ready) {
+    const float gpx = D_(0), gpy = D_(1), gA = D_(2), gB = D_(3), gC = D_(4), go = D_(5);
     const float p[3] = {R_(0), R_(1), R_(2)};
     float pv[4], clip[4];
     for (int i = 0; i < 4; ++i) {
@@ -128,7 +131,7 @@ __device__ __forceinline__ void backward_gaussian(const ViewBlock& sv, const flo
 #pragma unroll
         for (int k = 1; k < 16; ++k) raw += Y[k] * R_(kRowRest + (k - 1) + 15 * ch);
         raw += 0.5f;
-        gcol[ch] = raw < 0.0f ? 0.0f : d2[6 + ch];
+        gcol[ch] = raw < 0.0f ? 0.0f : D_(6 + ch);
     }
     float wsh[16];
 #pragma unroll
@@ -247,7 +250,7 @@ __device__ __forceinline__ void write_packed(const float (*tile)[kBwdPitch], flo
 // writes its slice of the packed layout (pos | log-scale | rot | f_dc | opacity | f_rest blocks, the
 // layout gs_scene_upload takes) with coalesced stores; invisible Gaussians get zeros.
 // Reads past the slice: counts are read in whole 16-byte units (the buffer holds roundup(N + 1, 8)
-// entries) and grad2d likewise (it holds 9N + 4 floats).
+// entries) and grad2d's opacity plane likewise (grad2d holds 9N + 4 floats).
 __global__ void __launch_bounds__(kBwdGroup, 6) k_preprocess_backward(const float* __restrict__ rows, uint32_t stride,
                                                                    uint32_t n, const ViewBlock* __restrict__ vb,
                                                                    const uint32_t* __restrict__ counts,
@@ -256,7 +259,8 @@ __global__ void __launch_bounds__(kBwdGroup, 6) k_preprocess_backward(const floa
     pdl_wait();
     static_assert(sizeof(ViewBlock) % 16 == 0, "the view block is copied in 16-byte units");
     __shared__ __align__(128) float s_rows[kRows][kBwdPitch];
-    __shared__ __align__(16) float s_d2[kBwdGroup * 9];
+    __shared__ __align__(16) float s_d2[kBwdGroup * 8];  // the slice's rows of grad2d
+    __shared__ __align__(16) float s_do[kBwdGroup];       // and its part of the opacity plane
     __shared__ __align__(16) uint32_t s_cnt[kBwdGroup];
     __shared__ __align__(16) ViewBlock sv;
     __shared__ __align__(8) uint64_t s_bar[2];  // [0]: view, counts, 2D gradients, geometry rows; [1]: f_rest rows
@@ -283,11 +287,11 @@ __global__ void __launch_bounds__(kBwdGroup, 6) k_preprocess_backward(const floa
     };
     if (lt == 0) {
         const uint32_t cnt_bytes = ((cnt + 3u) & ~3u) * 4u;
-        const uint32_t d2_bytes = (cnt * 36u + 15u) & ~15u;
-        mbar_expect_tx(&s_bar[0], (uint32_t)sizeof(ViewBlock) + cnt_bytes + d2_bytes + kRowRest * cols * 4u);
+        mbar_expect_tx(&s_bar[0], (uint32_t)sizeof(ViewBlock) + 2u * cnt_bytes + cnt * 32u + kRowRest * cols * 4u);
         bulk_g2s(&sv, vb, (uint32_t)sizeof(ViewBlock), &s_bar[0]);
         bulk_g2s(s_cnt, counts + g0, cnt_bytes, &s_bar[0]);
-        bulk_g2s(s_d2, grad2d + (size_t)9 * g0, d2_bytes, &s_bar[0]);
+        bulk_g2s(s_d2, grad2d + (size_t)8 * g0, cnt * 32u, &s_bar[0]);
+        bulk_g2s(s_do, grad2d + (size_t)8 * n + g0, cnt_bytes, &s_bar[0]);
         for (int r = 0; r < kRowRest; ++r)
             bulk_g2s(&s_rows[r][0], rows + (size_t)r * stride + g0, cols * 4u, &s_bar[0]);
         // the f_rest rows too, at once: with the Gaussians in scene order almost every slice holds a
@@ -303,11 +307,14 @@ __global__ void __launch_bounds__(kBwdGroup, 6) k_preprocess_backward(const floa
     if (any) {
         // the slice's 2D gradients are in shared memory now (every thread passed the copy's barrier):
         // clear them in global memory for the next raster backward, which only accumulates
-        for (uint32_t i = lt; i < 9u * cnt; i += kBwdGroup) grad2d[(size_t)9 * g0 + i] = 0.0f;
+        for (uint32_t i = lt; i < 2u * cnt; i += kBwdGroup)
+            reinterpret_cast<float4*>(grad2d)[(size_t)2 * g0 + i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (lt < cnt) grad2d[(size_t)8 * n + g0 + lt] = 0.0f;
         if (vis) {
             auto R_ = [&](int row) { return s_rows[row][lt]; };
             auto W_ = [&](int row, float v) { s_rows[row][lt] = v; };
-            backward_gaussian(sv, s_d2 + 9 * lt, R_, W_, [&]() { wait_bar(&s_bar[1]); });
+            auto D_ = [&](int k) { return k == 5 ? s_do[lt] : s_d2[8 * lt + kGradPlace[k]]; };
+            backward_gaussian(sv, D_, R_, W_, [&]() { wait_bar(&s_bar[1]); });
         } else {
             // every thread waits for the f_rest copies before it overwrites its column or leaves: no
             // bulk copy may still write into shared memory that is reused or released
@@ -364,11 +371,14 @@ __global__ void __launch_bounds__(kBwdGroup) k_preprocess_backward_multi(const f
             if (lt < 44) reinterpret_cast<uint32_t*>(&sv)[lt] = reinterpret_cast<const uint32_t*>(mv.view[v])[lt];
             __syncthreads();
             if (seen & (1u << v)) {
-                float* d2 = mv.grad2d[v] + (size_t)9 * g;
-                backward_gaussian(sv, d2, R_, W_, []() {});
+                float4* row = reinterpret_cast<float4*>(mv.grad2d[v]) + (size_t)2 * g;
+                float* d_op = mv.grad2d[v] + (size_t)8 * n + g;
+                const float4 lo = row[0], hi = row[1];
+                const float d2[9] = {lo.x, lo.y, hi.x, hi.y, hi.z, *d_op, lo.z, lo.w, hi.w};
+                backward_gaussian(sv, [&](int k) { return d2[k]; }, R_, W_, []() {});
                 // cleared for the next raster backward, which only accumulates
-#pragma unroll
-                for (int k = 0; k < 9; ++k) d2[k] = 0.0f;
+                row[0] = row[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                *d_op = 0.0f;
             }
         }
     }
@@ -381,6 +391,7 @@ __global__ void __launch_bounds__(kBwdGroup) k_preprocess_backward_multi(const f
 size_t preprocess_backward_multi_smem() { return (size_t)2 * kRows * kBwdPitch * sizeof(float); }
 
 void configure_backward_kernels() {
+    configure_raster_backward();
     cudaFuncSetAttribute(k_preprocess_backward_multi, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)preprocess_backward_multi_smem());
 }

@@ -109,6 +109,8 @@ __global__ void __launch_bounds__(TILE * TILE, raster_min_blocks<TILE, LAST>()) 
                 hit = box_meets(s_box[g0 + lane], rx0, rx1, ry0, ry1) &&
                       box_meets(s_diag[g0 + lane], rx0 + ry0, rx1 + ry1, rx0 - ry1, rx1 - ry0);
             uint32_t m = __ballot_sync(0xffffffffu, hit);
+            if (LAST && lane == 0u && out.hit_masks)  // the backward visits the same splats
+                out.hit_masks[warp * out.mask_pitch + hit_mask_base(start, tile) + ((i - start + g0) >> 5)] = m;
             while (m) {
                 const uint32_t j = g0 + (uint32_t)(__ffs(m) - 1);
                 m &= m - 1u;
