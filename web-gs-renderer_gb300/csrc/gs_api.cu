@@ -555,6 +555,7 @@ int gs_ctx_create(const gs_config* cfg, gs_ctx** out) {
     }
     if (cudaSetDevice(c.device) != cudaSuccess) return GS_ERR_CUDA;
     configure_sort_kernels();
+    configure_raster_kernels();
     configure_backward_kernels();
     gs_ctx* ctx = new gs_ctx();
     ctx->cfg = c;
@@ -942,7 +943,7 @@ int gs_get_debug(gs_ctx* ctx, const gs_debug* dbg) {
         std::vector<float> rec((size_t)n * kRecFloat4 * 4);
         if (n) GS_CK(cudaMemcpy(rec.data(), f.rec.p, rec.size() * 4, cudaMemcpyDeviceToHost));
         for (size_t g = 0; g < n; ++g) {
-            const float* r = rec.data() + g * 12;
+            const float* r = rec.data() + g * (kRecFloat4 * 4);
             if (dbg->pixel) { dbg->pixel[2 * g] = r[0]; dbg->pixel[2 * g + 1] = r[1]; }
             if (dbg->conic_opacity) {
                 dbg->conic_opacity[4 * g] = r[2];

@@ -43,16 +43,6 @@ __device__ __forceinline__ float tf32_head(float v) {
     return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u);
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
-
 // Predicated adds to global memory (no branch around them).
 __device__ __forceinline__ void red_add4_if(bool on, float* p, float x, float y, float z, float w) {
     asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n @q red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n}"

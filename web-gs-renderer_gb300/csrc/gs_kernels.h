@@ -8,11 +8,12 @@
 
 namespace gs {
 
-// Per-Gaussian raster record written by preprocess (three float4 per Gaussian):
+// Per-Gaussian raster record written by preprocess (four float4 per Gaussian, two 32-byte sectors):
 //   r0 = (pixel.x, pixel.y, conic.x, conic.y)
 //   r1 = (conic.z, opacity, color.r, color.g)
 //   r2 = (color.b, power cut-off below which alpha < 1/255 for sure, 0, 0)
-constexpr int kRecFloat4 = 3;
+//   r3 = half extents of the cull octagon along x, y, x + y, x - y (gs_raster_common.cuh)
+constexpr int kRecFloat4 = 4;
 
 // ---- scene layout -------------------------------------------------------------------------
 // packed (reference layout, preprocess.wgsl:16-24) -> rows of the structure-of-arrays layout.
@@ -153,8 +154,10 @@ struct RasterOut {
 // First word of a tile's groups in a plane: the tiles' starts grow with their index, so (start / 32 + tile)
 // leaves every tile ceil(length / 32) words of its own; a plane holds max_instance / 32 + tiles + 1.
 __host__ __device__ __forceinline__ size_t hit_mask_base(uint32_t start, uint32_t tile) { return (size_t)(start >> 5) + tile; }
-// ctl (optional) bounds every range by the sorted count; n bounds the Gaussian indices; order
+// configure_raster_kernels: kernel attributes, once per device. batch: a quarter of the range
+// positions culled per step (32 to 256). ctl (optional) bounds every range by the sorted count; n bounds the Gaussian indices; order
 // (optional) is the tile each CTA renders (launch_tile_order), else CTA i renders tile i.
+void configure_raster_kernels();
 void launch_raster(uint32_t tile, uint32_t batch, const uint32_t* ranges, const uint32_t* vals, const float4* rec,
                    uint32_t n, const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x,
                    uint32_t tiles_y, const RasterOut& out, const uint32_t* order, cudaStream_t s);

@@ -243,6 +243,10 @@ __device__ __forceinline__ bool preprocess_gaussian(uint32_t g, const ViewBlock&
         counts[g] = 0u;
         return true;
     }
+    // the pixels of the splat's tiles lie within its radius and a tile of its centre (and a pixel for the
+    // rounding of the sums)
+    rec[(size_t)kRecFloat4 * g + 3] =
+        cull_extents(pixx, pixy, conx, cony, conz, cut, (radius + (float)tile + 1.0f) * 1.00001f);
     // tile AABB, depth16, tilesTouched (:122-143)
     const float bminx = pixx - radius, bminy = pixy - radius;
     const float bmaxx = pixx + radius, bmaxy = pixy + radius;

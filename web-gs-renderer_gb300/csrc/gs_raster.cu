@@ -1,32 +1,41 @@
 // gs_raster.cu -- front-to-back alpha-blending tile rasterizer (src/shaders/raseter.wgsl:35-117).
 //
-// One CTA per tile, one thread per pixel; each warp owns an 8x4 block of the tile. The tile's
-// sorted range is walked in batches of BATCH splats: the CTA votes to stop once every pixel is done
-// (raseter.wgsl:54-68 as one __syncthreads_and) and stages the batch's records in shared memory
-// with one gather per splat. Every pixel then blends the batch in order with the pinned fp32
+// One thread per pixel; each warp owns an 8x4 block of a tile, a CTA up to 16x16 pixels (a 32x32 tile
+// takes four). Every pixel blends the splats of the tile's sorted range in order with the pinned fp32
 // semantics:
 //   power = fma(-0.5, fma(a*dx, dx, (c*dy)*dy), -((b*dx)*dy)); skip if power > 0
 //   alpha = min(0.99, o * exp(power));                         skip if alpha < 1/255
 //   testT = T * (1 - alpha);                                   done if testT < 1e-4
 //   C += colour * alpha * T (one fma per channel); T = testT
 //
-// Two exact shortcuts remove most of the work without changing a single output bit:
-//  * cut-off: a pixel whose power is below the splat's cut-off c_o = ln((1/255)/o) - 1e-3 is
-//    rejected without its alpha, since o*exp(power) < 1/255 is certain there (the 1e-3 margin is
-//    far beyond the rounding of exp, the product and logf); so alpha is only ever used where the
-//    raster's exp is defined (lanes of a hit form it anyway and discard it: no branch in a hit);
-//  * warp cull: when staging a splat, the CTA computes an octagon (the bounding box and the
-//    45-degree box) around the region of the tile where power >= c_o can hold
-//    (gs_raster_common.cuh gives the bound). Every warp tests its 8x4 pixel block against the 32
-//    octagons of a group in parallel (one per lane, one ballot) and walks only the splats whose
-//    octagon meets its block, in range order. A skipped splat would have been rejected by every
-//    pixel of the warp at "power < c_o" (or "power > 0"). Contributor counts are range positions, so
-//    skipping does not change them.
+// Cull. The CTA takes the range in steps (4 x raster_batch positions, one vote per step to stop once every
+// pixel is done, raseter.wgsl:54-68): one lane per splat tests the octagon around the region where
+// power >= c_o = ln((1/255)/o) - 1e-3 can hold (its half extents come with the record,
+// gs_raster_common.cuh) against the CTA's blocks, and ballots turn the answers into one word per warp
+// and 32 positions. A splat outside a block would have been rejected by each of its pixels, so walking only
+// the hits changes no output bit. Contributor counts are range positions, so skipping does not change
+// them.
 //
-// Full residency (2048 threads per SM, 32 registers; the few spilled bytes cost less than the lost
-// warps did), except for the instantiation that also tracks the contributor count (below).
+// Walk. From there a warp is on its own: it stages the records of its hits in a ring of its own by
+// asynchronous copies, 32 positions at a time, while it blends the hits staged before. A lane each lays
+// 16 to 32 hits out as pairs, and the arithmetic up to the blend (power, exp, alpha, 1 - alpha,
+// colour times alpha) runs on two splats at once by packed fp32 operations, which round each half like the
+// scalar ones; only the blend itself goes splat by splat, by predicated instructions. Below a power of -20
+// alpha is formed at -20, where every opacity's is under 1/255, so the cut-off need not travel with the hit.
 //
-// CTA i renders tile order[i]: the tiles listed by decreasing range length, so the longest tiles
+// What bounds it: shared-memory reads of the hits' nine values (a 16-byte read returns 512 bytes to a
+// warp, four cycles of the SM's 128 bytes), 52% of the time at 1M / 1080p, the fp32 pipe 51%, issue 65%;
+// more warps (40 or 48 per SM, at 48 or 40 registers) measured the same, 24 slower. Measured against one CTA
+// per tile that staged 256 splats between two barriers, computed the octagon per tile and splat and walked
+// the bits of its ballots at one splat per step (32 registers, 2048 threads per SM): 1M / 1080p
+// 189.5 -> 181.8 us (216M -> 146M warp instructions), 3M / 4K 1168 -> 1031, 250k / 1237x823 in 8x8 tiles
+// 105 -> 72, a close-up of 60k at 1600x900 212 -> 187, 16 views in 32x32 tiles 3906 -> 2432 in sum, a 300-tile
+// view of 100k 76 -> 50, 50k / 512x512 47.6 -> 35.6. On the way, 1M / 1080p: the pairs alone 211 us
+// (3 selects per blend instead of predicates, octagons per tile, a barrier per 256 positions), predicates
+// and steps of 1024 200, without the cut-off's reads 195.5, half extents from the preprocess and up to 32 hits
+// per step 181.8; the packed constants read from constant memory 191.
+//
+// Tiles start in order[]'s order: by decreasing range length, so the longest tiles
 // start first instead of forming the tail of the launch (with tiles in index order the clustered
 // scenes left about a third of the launch time to a few long tiles).
 #include "gs_kernels.h"
@@ -35,114 +44,230 @@
 namespace gs {
 namespace {
 
-// Residency: 2048 threads per SM (32 registers); the 16x16 instantiation that also tracks the
-// contributor count runs at 1536 (40 registers, no spills): 0.2705 -> 0.2683 ms per 1M / 1080p
-// differentiable frame, while the plain frame is fastest at full residency (0.2621 against 0.2683).
-template <int TILE, bool LAST>
-constexpr int raster_min_blocks() { return LAST && TILE == 16 ? 6 : 2048 / (TILE * TILE); }
+// Bits of the warps whose 8x4 block of the SUB x SUB pixels at (px0, py0) the octagon of a splat at (x, y)
+// with the half extents e (gs_raster_common.cuh) meets; all of them where no bound exists.
+template <int SUB>
+__device__ __forceinline__ uint32_t block_bits(float x, float y, const float4& e, float px0, float py0) {
+    constexpr int WX = SUB / 8, WY = SUB / 4;
+    const float x0 = x - e.x, x1 = x + e.x, y0 = y - e.y, y1 = y + e.y;
+    const float u = x + y, v = x - y, u0 = u - e.z, u1 = u + e.z, v0 = v - e.w, v1 = v + e.w;
+    uint32_t bits = 0;
+#pragma unroll
+    for (int by = 0; by < WY; ++by)
+#pragma unroll
+        for (int bx = 0; bx < WX; ++bx) {
+            const float rx0 = px0 + 8.0f * bx, rx1 = rx0 + 7.0f, ry0 = py0 + 4.0f * by, ry1 = ry0 + 3.0f;
+            const bool meets = (x1 >= rx0) & (x0 <= rx1) & (y1 >= ry0) & (y0 <= ry1) & (u1 >= rx0 + ry0) &
+                               (u0 <= rx1 + ry1) & (v1 >= rx0 - ry1) & (v0 <= rx1 - ry0);
+            bits |= meets ? 1u << (by * WX + bx) : 0u;
+        }
+    return e.x < __int_as_float(0x7f800000) ? bits : (1u << (WX * WY)) - 1u;
+}
 
-template <int TILE, int BATCH, bool LAST>
-__global__ void __launch_bounds__(TILE * TILE, raster_min_blocks<TILE, LAST>()) k_raster(const uint32_t* __restrict__ ranges,
-                                                        const uint32_t* __restrict__ vals,
-                                                        const float4* __restrict__ rec, uint32_t n,
-                                                        const FrameCtl* __restrict__ ctl, uint32_t width,
-                                                        uint32_t height, uint32_t tiles_x, RasterOut out,
-                                                        const uint32_t* __restrict__ order) {
+constexpr uint32_t kRing = 64;          // staged hits per warp (room for 32 more at kChunkMin + 16 pending)
+constexpr uint32_t kChunk = 32;         // most hits blended per step (one lane each lays them out in pairs)
+constexpr uint32_t kChunkMin = 16;      // fewest, until the tile's last
+constexpr uint32_t kMaxGroups = 32;     // groups of 32 range positions per cull step, at most
+
+// Shared memory of a warp: a ring of staged hits and the step's hits as pairs.
+struct RasterWarp {
+    float4 a[kRing];  // (x, y, conic.x, conic.y)
+    float4 b[kRing];  // (conic.z, opacity, r, g)
+    float4 c[kRing];  // (b, cut, range position, unused)
+    float4 pair[kChunk / 2][5];  // (x, x', y, y'), (A, A', -B, -B'), (C, C', o, o'), (r, r', g, g'),
+                                 // (b, b', position, position')
+};
+template <int TILE>
+struct RasterShared {
+    static constexpr int kSub = TILE < 16 ? TILE : 16;  // a CTA renders kSub x kSub pixels of a tile
+    static constexpr int kWarps = kSub * kSub / 32;
+    RasterWarp warp[kWarps];
+    uint32_t masks[kMaxGroups][kWarps];  // the step's hits per group and warp
+};
+
+// max that keeps a NaN. Below the floor no splat of any opacity reaches 1/255, and from it up o * exp(power)
+// stays normal for an opacity of at least 1/255.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+constexpr float kPowerFloor = -20.0f;
+
+// What a raster keeps besides the colours: nothing, the final transmittance, or that and the contributor
+// count (and, for a differentiable frame, the hit masks).
+constexpr int kKeepNothing = 0, kKeepT = 1, kKeepLast = 2;
+
+// One pixel's blend of one splat given its alpha, 1 - alpha and colour times alpha. No branch: the splat
+// counts unless power > 0, power < cut or alpha < 1/255 (a NaN power passes, as in the comparisons' plain
+// form), and blends if testT >= 1e-4, by predicated instructions (written out: as selects they cost three
+// more). T takes testT either way: once below 1e-4 it stays below, so nothing blends any more (a pixel
+// outside the image starts at 0); final_t is the transmittance after the last blend.
+template <int KEEP>
+__device__ __forceinline__ void blend_one(float power, float alpha, float one_minus, float ra, float ga,
+                                          float ba, uint32_t pos, float& T, float& cr, float& cg, float& cb,
+                                          float& final_t, uint32_t& last) {
+    const float testT = T * one_minus;
+#define GS_BLEND(EXTRA, F, L)                                                                                          \
+    asm("{\n .reg .pred in, blend;\n"                                                                            \
+        " setp.leu.f32 in, %6, 0f00000000;\n"                                                                    \
+        " setp.geu.and.f32 in, %7, %8, in;\n"                                                                    \
+        " setp.ge.and.f32 blend, %9, %10, in;\n"                                                                 \
+        " @blend fma.rn.f32 %1, %11, %0, %1;\n"                                                                  \
+        " @blend fma.rn.f32 %2, %12, %0, %2;\n"                                                                  \
+        " @blend fma.rn.f32 %3, %13, %0, %3;\n"                                                                  \
+        " @in mov.f32 %0, %9;\n" EXTRA "}"                                                                       \
+        : "+f"(T), "+f"(cr), "+f"(cg), "+f"(cb), F, L                                                              \
+        : "f"(power), "f"(alpha), "f"(kEpsilon), "f"(testT), "f"(kBlendThreshold), "f"(ra), "f"(ga),             \
+          "f"(ba), "r"(pos))
+    if constexpr (KEEP == kKeepNothing) {
+        float none;
+        uint32_t unset;
+        GS_BLEND("", "=f"(none), "=r"(unset));
+    } else if constexpr (KEEP == kKeepT) {
+        uint32_t unset;
+        GS_BLEND(" @blend mov.f32 %4, %9;\n", "+f"(final_t), "=r"(unset));
+    } else {
+        GS_BLEND(" @blend mov.f32 %4, %9;\n @blend mov.u32 %5, %14;\n", "+f"(final_t), "+r"(last));
+    }
+}
+#undef GS_BLEND
+
+template <int TILE, int KEEP>
+__global__ void __launch_bounds__(RasterShared<TILE>::kWarps * 32, 32 / RasterShared<TILE>::kWarps)
+k_raster(const uint32_t* __restrict__ ranges, const uint32_t* __restrict__ vals, const float4* __restrict__ rec,
+         uint32_t n, const FrameCtl* __restrict__ ctl, uint32_t width, uint32_t height, uint32_t tiles_x, RasterOut out,
+         const uint32_t* __restrict__ order, uint32_t step) {
     pdl_wait();
-    constexpr int THREADS = TILE * TILE;
-    constexpr int WX = TILE / 8;  // warps across the tile
-    __shared__ float4 s_a[BATCH];    // (x, y, conic.x, conic.y)
-    __shared__ float4 s_b[BATCH];    // (conic.z, opacity, r, g)
-    __shared__ float2 s_c[BATCH];    // (b, cut)
-    __shared__ float4 s_box[BATCH];  // cull box (x0, x1, y0, y1)
-    __shared__ float4 s_diag[BATCH];  // its 45-degree box (u0, u1, v0, v1), u = x + y, v = x - y
+    constexpr bool LAST = KEEP == kKeepLast;
+    constexpr uint32_t kSub = RasterShared<TILE>::kSub, kWarps = RasterShared<TILE>::kWarps, kThreads = 32u * kWarps;
+    constexpr uint32_t kSubs = TILE / kSub;  // CTAs across the tile
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    RasterShared<TILE>& cta = *reinterpret_cast<RasterShared<TILE>*>(s_raw);
 
-    const uint32_t tile = order ? order[blockIdx.x] : blockIdx.x;
-    const uint32_t tx = tile % tiles_x, ty = tile / tiles_x;
+    const uint32_t sub = blockIdx.x % (kSubs * kSubs), at = blockIdx.x / (kSubs * kSubs);
+    const uint32_t tile = order ? order[at] : at;
+    const uint32_t px0 = (tile % tiles_x) * TILE + kSub * (sub % kSubs), py0 = (tile / tiles_x) * TILE + kSub * (sub / kSubs);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t bx0 = tx * TILE + 8u * (warp % WX), by0 = ty * TILE + 4u * (warp / WX);
-    const uint32_t x = bx0 + (lane & 7u), y = by0 + (lane >> 3);
+    RasterWarp& sh = cta.warp[warp];
+    const uint32_t bx = 8u * (warp % (kSub / 8u)), by = 4u * (warp / (kSub / 8u));  // the warp's block
+    const uint32_t x = px0 + bx + (lane & 7u), y = py0 + by + (lane >> 3);
+    // plane of the hit masks: the block's number in the tile, row by row
+    const uint32_t plane = ((kSub * (sub / kSubs) + by) / 4u) * (TILE / 8u) + (kSub * (sub % kSubs) + bx) / 8u;
     const bool inside = x < width && y < height;
-    bool done = !inside;
     const uint2 range = reinterpret_cast<const uint2*>(ranges)[tile];
     // a range past the sorted count can only come from a timed-out sort: clamp it
     const uint32_t end = ctl ? min(range.y, ctl->sorted_count) : range.y;
     const uint32_t start = range.x;
-    const float fx = (float)x, fy = (float)y;
-    const float rx0 = (float)bx0, rx1 = (float)(bx0 + 7u), ry0 = (float)by0, ry1 = (float)(by0 + 3u);
-    const float tx0 = (float)(tx * TILE), tx1 = (float)(tx * TILE + TILE - 1u);
-    const float ty0 = (float)(ty * TILE), ty1 = (float)(ty * TILE + TILE - 1u);
+    const float2 nfx = both(-(float)x), nfy = both(-(float)y);
 
-    float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
+    float T = inside ? 1.0f : 0.0f, final_t = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
     uint32_t last = 0;
+    uint32_t head = 0, ready = 0, tail = 0;  // hits blended, staged for certain, staged or on their way
+    bool over = false;                       // every pixel of the warp is done
 
-    for (uint32_t i = start; i < end; i += BATCH) {
-        if (__syncthreads_and(done)) break;
-        for (uint32_t j = threadIdx.x; j < (uint32_t)BATCH; j += THREADS) {
-            if (i + j < end) {
-                const uint32_t g = vals[i + j];
-                if (g < n) {
-                    const float4 r0 = __ldg(rec + (size_t)kRecFloat4 * g);
-                    const float4 r1 = __ldg(rec + (size_t)kRecFloat4 * g + 1);
-                    const float4 r2 = __ldg(rec + (size_t)kRecFloat4 * g + 2);
-                    s_a[j] = r0;
-                    s_b[j] = r1;
-                    s_c[j] = make_float2(r2.x, r2.y);
-                    s_box[j] = cull_box(r0.x, r0.y, r0.z, r0.w, r1.x, r2.y, tx0, tx1, ty0, ty1, s_diag[j]);
-                } else {  // only after a timed-out sort: a splat that never blends
-                    const float inf = __int_as_float(0x7f800000);
-                    s_a[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    s_b[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    s_c[j] = make_float2(0.0f, inf);
-                    s_box[j] = make_float4(inf, -inf, inf, -inf);
-                    s_diag[j] = s_box[j];
-                }
+    // blends the next cnt (at most kChunk) staged hits
+    auto blend = [&](uint32_t cnt) {
+        {
+            const uint32_t slot = (head + lane) % kRing;
+            float4 a = sh.a[slot], b = sh.b[slot], c = sh.c[slot];
+            float* q = reinterpret_cast<float*>(sh.pair[lane >> 1]) + (lane & 1u);
+            // past the hits (where the ring may hold anything) alpha is 0; so it is below a positive
+            // cut-off, where the opacity itself is under 1/255
+            if (lane >= cnt) a = b = c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (c.y > 0.0f) b.y = 0.0f;
+            q[0] = a.x; q[2] = a.y; q[4] = a.z; q[6] = -a.w;
+            q[8] = b.x; q[10] = b.y; q[12] = b.z; q[14] = b.w;
+            q[16] = c.x;
+            if (LAST) q[18] = c.z;
+        }
+        __syncwarp();
+        const uint32_t pairs = (cnt + 1u) / 2u;
+#pragma unroll 2
+        for (uint32_t k = 0; k < pairs; ++k) {
+            const float4 p0 = sh.pair[k][0], p1 = sh.pair[k][1], p2 = sh.pair[k][2], p3 = sh.pair[k][3];
+            float2 p4, pos = make_float2(0.0f, 0.0f);
+            if (LAST) {
+                const float4 v = sh.pair[k][4];
+                p4 = make_float2(v.x, v.y);
+                pos = make_float2(v.z, v.w);
+            } else {
+                p4 = *reinterpret_cast<const float2*>(&sh.pair[k][4]);
             }
+            const float2 dx = __fadd2_rn(make_float2(p0.x, p0.y), nfx), dy = __fadd2_rn(make_float2(p0.z, p0.w), nfy);
+            const float2 q = __ffma2_rn(__fmul2_rn(make_float2(p1.x, p1.y), dx), dx,
+                                        __fmul2_rn(__fmul2_rn(make_float2(p2.x, p2.y), dy), dy));
+            const float2 power = __ffma2_rn(both(-0.5f), q, __fmul2_rn(__fmul2_rn(make_float2(p1.z, p1.w), dx), dy));
+            const float2 op = raster_alpha_unclamped2(make_float2(p2.z, p2.w), make_float2(max_nan(power.x, kPowerFloor), max_nan(power.y, kPowerFloor)));
+            const float2 alpha = make_float2(fminf(kAlphaClamp, op.x), fminf(kAlphaClamp, op.y));
+            const float2 om = __ffma2_rn(alpha, both(-1.0f), both(1.0f));
+            const float2 ra = __fmul2_rn(make_float2(p3.x, p3.y), alpha), ga = __fmul2_rn(make_float2(p3.z, p3.w), alpha);
+            const float2 ba = __fmul2_rn(p4, alpha);
+            blend_one<KEEP>(power.x, alpha.x, om.x, ra.x, ga.x, ba.x, __float_as_uint(pos.x), T, cr, cg, cb, final_t, last);
+            blend_one<KEEP>(power.y, alpha.y, om.y, ra.y, ga.y, ba.y, __float_as_uint(pos.y), T, cr, cg, cb, final_t, last);
+        }
+        head += cnt;
+        over = __all_sync(0xffffffffu, T < kBlendThreshold);
+        __syncwarp();
+    };
+
+    for (uint32_t i = start; i < end; i += step) {
+        if (__syncthreads_and(over)) break;
+        const uint32_t cnt = min(step, end - i);
+        // cull: each splat's octagon against the tile's blocks, one word per warp and 32 positions
+        for (uint32_t j = threadIdx.x; j < (cnt + 31u & ~31u); j += kThreads) {
+            uint32_t bits = 0;
+            const uint32_t g = j < cnt ? vals[i + j] : n;
+            if (g < n) {  // always, unless the sort timed out
+                const float2 c = __ldg(reinterpret_cast<const float2*>(rec + (size_t)kRecFloat4 * g));
+                bits = block_bits<kSub>(c.x, c.y, __ldg(rec + (size_t)kRecFloat4 * g + 3), (float)px0, (float)py0);
+            }
+            uint32_t word = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < kWarps; ++w) {
+                const uint32_t b = __ballot_sync(0xffffffffu, bits >> w & 1u);
+                word = lane == w ? b : word;
+            }
+            if (lane < kWarps) cta.masks[j >> 5][lane] = word;
         }
         __syncthreads();
-        const uint32_t cnt = min((uint32_t)BATCH, end - i);
-        const uint32_t pos0 = i - start + 1u;  // contributor count of the batch's first splat
-        for (uint32_t g0 = 0; g0 < cnt; g0 += 32u) {
-            if (__all_sync(0xffffffffu, done)) break;
-            bool hit = false;
-            if (g0 + lane < cnt)
-                hit = box_meets(s_box[g0 + lane], rx0, rx1, ry0, ry1) &&
-                      box_meets(s_diag[g0 + lane], rx0 + ry0, rx1 + ry1, rx0 - ry1, rx1 - ry0);
-            uint32_t m = __ballot_sync(0xffffffffu, hit);
-            if (LAST && lane == 0u && out.hit_masks)  // the backward visits the same splats
-                out.hit_masks[warp * out.mask_pitch + hit_mask_base(start, tile) + ((i - start + g0) >> 5)] = m;
-            while (m) {
-                const uint32_t j = g0 + (uint32_t)(__ffs(m) - 1);
-                m &= m - 1u;
-                // no branch in a hit: every lane forms alpha and the blend, and the rejections (pixel
-                // done, power > 0, power below the cut-off, alpha < 1/255, termination) only select
-                // what is kept. Nearly every hit has lanes on both sides of them, so the branches
-                // only added their divergence and reconvergence (raster of the 1M / 1080p frame
-                // 0.2510 -> 0.2417 ms, 0.2580 -> 0.2458 ms with the contributor count; with a branch
-                // for the rejections by power and selects after it, slower). A rejected lane's exp
-                // may be of any argument; its value is discarded.
-                const float4 a = s_a[j];
-                const float2 c = s_c[j];
-                const float4 b = s_b[j];
-                const float dx = a.x - fx, dy = a.y - fy;
-                const float power = __fmaf_rn(-0.5f, __fmaf_rn(a.z * dx, dx, (b.x * dy) * dy), -((a.w * dx) * dy));
-                const bool in = !(done || power > 0.0f || power < c.y);
-                const float alpha = fminf(kAlphaClamp, raster_alpha_unclamped(b.y, power));
-                const float testT = T * (1.0f - alpha);
-                const bool faint = alpha < kEpsilon;
-                const bool stop = in && !faint && testT < kBlendThreshold;
-                const bool blend = in && !faint && !stop;
-                done = done || stop;
-                const float wr = __fmaf_rn(b.z * alpha, T, cr), wg = __fmaf_rn(b.w * alpha, T, cg);
-                const float wb = __fmaf_rn(c.x * alpha, T, cb);
-                cr = blend ? wr : cr;
-                cg = blend ? wg : cg;
-                cb = blend ? wb : cb;
-                T = blend ? testT : T;
-                if (LAST && blend) last = pos0 + j;
+        if (over) continue;
+        const uint32_t groups = (cnt + 31u) / 32u;
+        const uint32_t words = lane < groups ? cta.masks[lane][warp] : 0u;
+        if (LAST && lane < groups && out.hit_masks)  // the backward visits the same splats
+            out.hit_masks[plane * out.mask_pitch + hit_mask_base(start, tile) + ((i - start) >> 5) + lane] = words;
+        uint32_t group = 0, m = 0, g = n;
+        // the next group with hits; its Gaussian indices are loaded while the group before it is staged
+        auto next_group = [&]() {
+            m = 0;
+            while (group < groups && (m = __shfl_sync(0xffffffffu, words, group)) == 0u) ++group;
+            if (m >> lane & 1u) g = vals[i + 32u * group + lane];
+        };
+        next_group();
+        while (m != 0u && !over) {
+            while (m != 0u && tail - head + __popc(m) <= kRing) {
+                if (m >> lane & 1u) {
+                    const uint32_t slot = (tail + __popc(m & ((1u << lane) - 1u))) % kRing;
+                    const float4* r = rec + (size_t)kRecFloat4 * g;
+                    cp_async16(&sh.a[slot], r);
+                    cp_async16(&sh.b[slot], r + 1);
+                    cp_async8(&sh.c[slot], r + 2);
+                    if (LAST) sh.c[slot].z = __uint_as_float(i - start + 32u * group + lane + 1u);
+                }
+                tail += __popc(m);
+                ++group;
+                next_group();
             }
+            cp_async_commit();
+            cp_async_wait<1>();
+            __syncwarp();
+            if (ready - head >= kChunkMin) blend(min(kChunk, ready - head) & ~1u);
+            ready = tail;
         }
     }
+    cp_async_wait<0>();
+    __syncwarp();
+    while (head < tail && !over) blend(min(kChunk, tail - head));
     if (!inside) return;
     const size_t p = (size_t)y * width + x;
     if (out.rgb) {
@@ -150,7 +275,7 @@ __global__ void __launch_bounds__(TILE * TILE, raster_min_blocks<TILE, LAST>()) 
         out.rgb[3 * p + 1] = cg;
         out.rgb[3 * p + 2] = cb;
     }
-    if (out.final_t) out.final_t[p] = T;
+    if (KEEP != kKeepNothing && out.final_t) out.final_t[p] = final_t;
     if (LAST) out.n_contrib[p] = last;
     if (out.rgba8) {
         const uint32_t r8 = (uint32_t)(fminf(fmaxf(cr, 0.0f), 1.0f) * 255.0f + 0.5f);
@@ -160,38 +285,44 @@ __global__ void __launch_bounds__(TILE * TILE, raster_min_blocks<TILE, LAST>()) 
     }
 }
 
-template <int TILE, int BATCH>
-void launch_batch(const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n, const FrameCtl* ctl,
-                  uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y, const RasterOut& out,
-                  const uint32_t* order, cudaStream_t s) {
-    const dim3 grid(tiles_x * tiles_y), block(TILE * TILE);
-    // the contributor count is tracked only when it is written (a differentiable forward): the
-    // plain frame's raster drops its register and update (0.509 -> 0.499 ms per 1M / 1080p frame)
-    if (out.n_contrib)
-        launch_pdl(k_raster<TILE, BATCH, true>, grid, block, s, ranges, vals, rec, n, ctl, width, height, tiles_x, out,
-                   order);
-    else
-        launch_pdl(k_raster<TILE, BATCH, false>, grid, block, s, ranges, vals, rec, n, ctl, width, height, tiles_x, out,
-                   order);
+template <int TILE>
+void launch_tile(uint32_t step, const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n,
+                 const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
+                 const RasterOut& out, const uint32_t* order, cudaStream_t s) {
+    constexpr uint32_t kSubs = TILE / RasterShared<TILE>::kSub;
+    const dim3 grid(tiles_x * tiles_y * kSubs * kSubs), block(RasterShared<TILE>::kWarps * 32);
+    const size_t smem = sizeof(RasterShared<TILE>);
+    auto launch = [&](auto kernel) {
+        launch_pdl_smem(kernel, grid, block, smem, s, ranges, vals, rec, n, ctl, width, height, tiles_x, out, order, step);
+    };
+    if (out.n_contrib) launch(k_raster<TILE, kKeepLast>);
+    else if (out.final_t) launch(k_raster<TILE, kKeepT>);
+    else launch(k_raster<TILE, kKeepNothing>);
 }
 
 template <int TILE>
-void launch_tile(uint32_t batch, const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n,
-                 const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
-                 const RasterOut& out, const uint32_t* order, cudaStream_t s) {
-    switch (batch) {
-        case 32: launch_batch<TILE, 32>(ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s); break;
-        case 64: launch_batch<TILE, 64>(ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s); break;
-        case 128: launch_batch<TILE, 128>(ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s); break;
-        default: launch_batch<TILE, 256>(ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s); break;
-    }
+void configure_tile() {
+    auto configure = [](auto kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RasterShared<TILE>));
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    };
+    configure(k_raster<TILE, kKeepNothing>);
+    configure(k_raster<TILE, kKeepT>);
+    configure(k_raster<TILE, kKeepLast>);
 }
 
 }  // namespace
 
+void configure_raster_kernels() {
+    configure_tile<8>();
+    configure_tile<16>();
+    configure_tile<32>();
+}
+
 void launch_raster(uint32_t tile, uint32_t batch, const uint32_t* ranges, const uint32_t* vals, const float4* rec,
                    uint32_t n, const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x,
                    uint32_t tiles_y, const RasterOut& out, const uint32_t* order, cudaStream_t s) {
+    batch *= 4u;  // positions per cull step (128 to 1024, a multiple of 32): most tiles need one step
     if (tile == 8) launch_tile<8>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s);
     else if (tile == 32) launch_tile<32>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s);
     else launch_tile<16>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s);

@@ -1,17 +1,18 @@
 // gs_raster_common.cuh -- pieces shared by the forward raster and its backward: the pinned exp on
-// the raster's argument range and the conservative per-warp cull of staged splats.
+// the raster's argument range and the conservative cull of splats against pixel blocks.
 //
 // Cull. For a splat with conic (a, b, c) and cut-off c_o = ln((1/255)/o) - 1e-3, a pixel can only
 // pass "power >= c_o" where Q(d) = a dx^2 + 2b dx dy + c dy^2 <= K', K' = -2 c_o plus the worst
-// rounding error of the pinned power formula anywhere in the tile (16 eps times S_max, the sum of
-// the absolute terms bounded over the tile). The cull box is the bounding box of {Q <= K'}, with
+// rounding error of the pinned power formula anywhere in the splat's tiles (16 eps times S_max, the sum
+// of the absolute terms bounded over them). The cull box is the bounding box of {Q <= K'}, with
 // det = ac - b^2 taken at its lower rounding bound; its 45-degree box bounds u = x + y and v = x - y
 // over the same region (half-extents sqrt(K' (a + c -+ 2b) / det)), and the two together form an
 // octagon around the ellipse. A splat whose octagon misses a warp's pixel block would have been
 // rejected by every pixel of the block at "power < c_o" (or "power > 0"), so skipping it changes no
 // output bit. Splats whose region cannot be bounded safely (non-positive-definite or non-finite
 // values) are never culled. Against the box alone the octagon removes 13.5% of the (8x4 block,
-// splat) hits of the 1M / 1080p frame and 10.9% of the (8x8 block, splat) hits.
+// splat) hits of the 1M / 1080p frame. The half extents are the preprocess's: once per Gaussian, not
+// once per tile that it touches.
 #pragma once
 #include "gs_common.cuh"
 
@@ -64,27 +65,39 @@ __device__ __forceinline__ float raster_alpha_unclamped(float o, float x) {
     return __int_as_float(__float_as_int(__fmul_rn(o, p)) + (__float_as_int(t) << 23));
 }
 
+// raster_alpha_unclamped of two splats at once: the packed fp32 operations round each half like the scalar
+// ones, so the bits are the same; every polynomial step is one issued instruction instead of two.
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 raster_alpha_unclamped2(float2 o, float2 x) {
+    const float2 t = __ffma2_rn(x, both(0x1.715476p+0f), both(12582912.0f));
+    const float2 n = __fadd2_rn(t, both(-12582912.0f));
+    const float2 r = __ffma2_rn(n, both(-0x1.62e43p-1f), x);
+    float2 p = both(0x1.6c350cp-10f);
+    p = __ffma2_rn(p, r, both(0x1.1246dap-7f));
+    p = __ffma2_rn(p, r, both(0x1.555638p-5f));
+    p = __ffma2_rn(p, r, both(0x1.55547ep-3f));
+    p = __ffma2_rn(p, r, both(0x1.fffffep-2f));
+    p = __ffma2_rn(p, r, both(1.0f));
+    p = __ffma2_rn(p, r, both(1.0f));
+    const float2 op = __fmul2_rn(o, p);
+    return make_float2(__int_as_float(__float_as_int(op.x) + (__float_as_int(t.x) << 23)),
+                       __int_as_float(__float_as_int(op.y) + (__float_as_int(t.y) << 23)));
+}
+
 __device__ __forceinline__ bool finite_f(float v) { return fabsf(v) <= 3.0e38f; }
 
-// Conservative box (x0, x1, y0, y1) for the tile [tx0,tx1] x [ty0,ty1], and in diag its 45-degree
-// box (u0, u1, v0, v1): (+inf, -inf, +inf, -inf) when no pixel can pass, (-inf, +inf, -inf, +inf)
-// when no safe bound exists. A warp block [rx0, rx1] x [ry0, ry1] spans u in [rx0 + ry0, rx1 + ry1]
-// and v in [rx0 - ry1, rx1 - ry0] (exact: integer coordinates).
-__device__ __forceinline__ float4 cull_box(float x, float y, float a, float b, float c, float cut, float tx0,
-                                           float tx1, float ty0, float ty1, float4& diag) {
+// Half extents of a splat's octagon along x, y, u = x + y and v = x - y, for pixels within `reach` of its
+// centre on either axis: -inf (all four) when no pixel can pass, +inf when no safe bound exists. A pixel block
+// [rx0, rx1] x [ry0, ry1] spans u in [rx0 + ry0, rx1 + ry1] and v in [rx0 - ry1, rx1 - ry0] (exact:
+// integer coordinates).
+__device__ __forceinline__ float4 cull_extents(float x, float y, float a, float b, float c, float cut, float reach) {
     const float inf = __int_as_float(0x7f800000);
-    const float4 keep_all = make_float4(-inf, inf, -inf, inf);
-    diag = keep_all;
+    const float4 keep_all = make_float4(inf, inf, inf, inf);
     if (!(finite_f(x) && finite_f(y) && finite_f(a) && finite_f(b) && finite_f(c)) || cut != cut) return keep_all;
     if (!(a > 0.0f) || !(c > 0.0f)) return keep_all;
-    const float dxm = fmaxf(fabsf(x - tx0), fabsf(x - tx1));
-    const float dym = fmaxf(fabsf(y - ty0), fabsf(y - ty1));
-    const float smax = (a * dxm * dxm + c * dym * dym + 2.0f * fabsf(b) * dxm * dym) * 1.01f;
+    const float smax = (a + c + 2.0f * fabsf(b)) * reach * reach * 1.01f;
     if (!finite_f(smax)) return keep_all;
-    if (cut > 0.0f) {  // power <= 0 < cut everywhere
-        diag = make_float4(inf, -inf, inf, -inf);
-        return diag;
-    }
+    if (cut > 0.0f) return make_float4(-inf, -inf, -inf, -inf);  // power <= 0 < cut everywhere
     const float ac = a * c, bb = b * b;
     const float det_lo = (ac - bb) - 4.0f * 0x1p-24f * (ac + bb);
     if (!(det_lo > 0.0f)) return keep_all;
@@ -100,16 +113,10 @@ __device__ __forceinline__ float4 cull_box(float x, float y, float a, float b, f
     const float su = (apc - b2) + 4.0f * 0x1p-24f * (apc + fabsf(b2));
     const float sv = (apc + b2) + 4.0f * 0x1p-24f * (apc + fabsf(b2));
     const float wu = __fdividef(k * su, det_lo), wv = __fdividef(k * sv, det_lo);
-    const float u = x + y, v = x - y;
-    const float hu = wu * rsqrtf(wu) * 1.00001f + 1.0e-3f + fabsf(u) * 0x1p-22f;
-    const float hv = wv * rsqrtf(wv) * 1.00001f + 1.0e-3f + fabsf(v) * 0x1p-22f;
-    if (finite_f(hu) && finite_f(hv) && su > 0.0f && sv > 0.0f) diag = make_float4(u - hu, u + hu, v - hv, v + hv);
-    return make_float4(x - hx, x + hx, y - hy, y + hy);
-}
-
-// Whether the box meets the pixel block [rx0,rx1] x [ry0,ry1].
-__device__ __forceinline__ bool box_meets(const float4& box, float rx0, float rx1, float ry0, float ry1) {
-    return box.y >= rx0 && box.x <= rx1 && box.w >= ry0 && box.z <= ry1;
+    const float hu = wu * rsqrtf(wu) * 1.00001f + 1.0e-3f + fabsf(x + y) * 0x1p-22f;
+    const float hv = wv * rsqrtf(wv) * 1.00001f + 1.0e-3f + fabsf(x - y) * 0x1p-22f;
+    const bool diagonal = finite_f(hu) && finite_f(hv) && su > 0.0f && sv > 0.0f;
+    return make_float4(hx, hy, diagonal ? hu : inf, diagonal ? hv : inf);
 }
 
 }  // namespace gs
