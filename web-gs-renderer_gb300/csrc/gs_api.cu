@@ -3,7 +3,7 @@
 // Replaces the reference Renderer (src/renderer/renderer.js): the context owns one CUDA stream and
 // per-view frame state (buffers sized from count * MAX_INSTANCE_FACTOR like renderer.js:531-577,
 // grown on demand and kept). gs_forward sequences the passes of renderer.js:822-932 on that stream,
-// replayed from one CUDA graph per (scene, resolution, output set); gs_forward_batch captures many
+// replayed from a CUDA graph while scene, resolution and output set stay the same; gs_forward_batch captures many
 // views, forked over side streams, into one graph. No pass reads a count back to the host: the
 // instance count travels in FrameCtl, which every later kernel reads on the device (the role of the
 // reference's indirect dispatch, indirect_arg.wgsl).
@@ -181,6 +181,7 @@ struct gs_ctx {
     // graph caches
     cudaGraphExec_t exec = nullptr, exec_batch = nullptr;
     GraphKey key, key_batch;
+    GraphKey last_key;  // of the last frame that could have come from a graph
 
     // pinned view blocks: a frame's H2D copy reads a slot that is not rewritten before the copy has
     // completed (slot_done), so frames never block the host
@@ -510,6 +511,7 @@ int capture_and_launch(gs_ctx* ctx, cudaGraphExec_t* exec, GraphKey* cached, con
 }
 
 void drop_graphs_of_scene(gs_ctx* ctx, const gs_scene* scene) {
+    ctx->last_key = GraphKey{};
     auto uses = [&](const GraphKey& k) { return std::find(k.ptrs.begin(), k.ptrs.end(), scene) != k.ptrs.end(); };
     if (ctx->exec && uses(ctx->key)) {
         cudaGraphExecDestroy(ctx->exec);
@@ -733,8 +735,19 @@ int gs_forward(gs_ctx* ctx, const gs_scene* scene, const gs_view* view, const gs
         k.ptrs = {scene, a.out.rgba8, a.out.rgb, a.out.final_t, a.out.n_contrib};
         k.dims = {a.n, a.w, a.h};
         k.alloc_gen = ctx->alloc_gen;
-        rc = capture_and_launch(ctx, &ctx->exec, &ctx->key, k, {&f}, {a});
-        if (rc != GS_OK) return rc;
+        // a graph is made for the second frame in a row of the same scene, size and outputs: capturing and
+        // instantiating one costs the host about 200 us, launching the frame's ten kernels about 25. A context
+        // that goes through views of different sizes (six views of three sizes, 400k Gaussians: 1190 -> 860 us) never pays
+        // for a graph it would not replay, and a single frame comes out sooner; a viewer replays from its
+        // third frame on.
+        const bool again = k == ctx->last_key;
+        if (!again) ctx->last_key = k;
+        if (again || (ctx->exec && k == ctx->key)) {
+            rc = capture_and_launch(ctx, &ctx->exec, &ctx->key, k, {&f}, {a});
+            if (rc != GS_OK) return rc;
+        } else {
+            enqueue_frame(ctx, f, a, ctx->stream, false);
+        }
     } else {
         enqueue_frame(ctx, f, a, ctx->stream, profile);
     }
