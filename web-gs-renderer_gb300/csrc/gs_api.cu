@@ -380,7 +380,7 @@ void enqueue_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a, cudaStream_t s, bo
         const uint32_t split = p * bits >= 16u && w / 2u >= 2u ? w / 2u : 0u;
         launch_onesweep(bits, f.keys[cur].p, f.vals[cur].p, f.keys[cur ^ 1].p, f.vals[cur ^ 1].p, &ctl->sorted_count,
                         0, a.max_instance, p * bits, radix - 1u, ctl->hist + p * radix, ctl, f.flags.p, 1 + p, 0, s,
-                        ctx->cfg.sort_block, split, p > 0,  // the emit right before the first pass writes its inputs
+                        ctx->cfg.sort_block, split,
                         p + 1 == a.passes ? f.ranges.p : nullptr, a.tiles_x * a.tiles_y);  // the last pass: ranges
         cur ^= 1;
     }

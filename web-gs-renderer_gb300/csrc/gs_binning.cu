@@ -147,16 +147,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
     __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
     __shared__ uint32_t s_part, s_excl, s_seq;
 
-    // the ticket counter and the sequence number were set by the frame's first kernel, two launches
-    // back: the partition is taken before the wait for the preprocess, whose counts are read after it
     const uint32_t tid = threadIdx.x;
+    const uint32_t radix = 1u << digit_bits;
+    for (uint32_t i = tid; i < passes * radix; i += kScanThreads) s_hist[i] = 0u;
+    pdl_wait();  // also for the ticket counter, set two kernels back: see k_onesweep
     if (tid == 0) {
         s_part = atomicAdd(&ctl->tickets[slot], 1u);
         s_seq = ctl->seq + slot;
     }
-    const uint32_t radix = 1u << digit_bits;
-    for (uint32_t i = tid; i < passes * radix; i += kScanThreads) s_hist[i] = 0u;
-    pdl_wait();
     __syncthreads();
     const uint32_t part = s_part, seq = s_seq;
     const uint32_t entries = n + 1u;
@@ -443,12 +441,11 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
                                                            const uint32_t* n_dev, uint32_t n_host, uint32_t shift,
                                                            uint32_t dmask, const uint32_t* __restrict__ hist,
                                                            FrameCtl* ctl, uint64_t* flags, uint32_t slot,
-                                                           uint32_t early, uint32_t* __restrict__ ranges,
-                                                           uint32_t tiles) {
-    // early: n, the histogram and the ticket counter were written before the previous kernel, so
-    // each CTA takes its first partition and computes the digit bases before waiting for that
-    // kernel (only the keys and values it wrote are read after the wait)
-    if (!early) pdl_wait();
+                                                           uint32_t* __restrict__ ranges, uint32_t tiles) {
+    // Nothing in global memory is read before the wait, not even what was written two kernels back (n, the
+    // histogram): a pass that took its ticket and digit bases early saw an unfinished histogram now and
+    // then when twenty views' sorts ran side by side in a graph (about 1 view in 300).
+    pdl_wait();
     constexpr uint32_t RADIX = 1u << BITS;
     const uint32_t MASK = dmask & (RADIX - 1u);  // digit mask of this pass (narrower on a last partial digit)
     constexpr uint32_t WARPS = kSortThreads / 32;
@@ -471,7 +468,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
     if (blockIdx.x >= nparts) return;
 
     if (tid == 0) s_seq = ctl->seq + slot;
-    bool have_bases = false, waited = early == 0u;
+    bool have_bases = false;
 
     while (true) {
         __syncthreads();
@@ -486,10 +483,6 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
             const uint32_t ex = block_exclusive_scan<kSortThreads>(h, s_warp, &tot);
             if (tid < RADIX) s_gbase[tid] = ex;
             have_bases = true;
-        }
-        if (!waited) {
-            pdl_wait();
-            waited = true;
         }
         const uint32_t base = part * PART;
         const uint32_t valid_n = min(PART, n - base);
@@ -790,7 +783,7 @@ void configure_sort_kernels() {
 void launch_onesweep(uint32_t digit_bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                      uint32_t* vals_out, const uint32_t* n_dev, uint32_t n_host, uint32_t max_n, uint32_t shift,
                      uint32_t dmask, const uint32_t* hist, FrameCtl* ctl, uint64_t* flags, uint32_t slot,
-                     int grid_cap, cudaStream_t s, uint32_t block, uint32_t split, bool early, uint32_t* ranges,
+                     int grid_cap, cudaStream_t s, uint32_t block, uint32_t split, uint32_t* ranges,
                      uint32_t tiles) {
     const bool small = block == kSortPartitionMin;
     const uint32_t part = small ? kSortPartitionMin : kSortPartition;
@@ -800,7 +793,7 @@ void launch_onesweep(uint32_t digit_bits, const uint32_t* keys_in, const uint32_
     if (parts == 0) parts = 1;
 #define GS_ONESWEEP(B, I, S)                                                                                      \
     launch_pdl(k_onesweep<B, I, S>, dim3(parts), dim3(kSortThreads), s, keys_in, vals_in, keys_out, vals_out, n_dev, \
-               n_host, shift, dmask, hist, ctl, flags, slot, early ? 1u : 0u, ranges, tiles)
+               n_host, shift, dmask, hist, ctl, flags, slot, ranges, tiles)
 #define GS_ONESWEEP_SPLIT(I)                             \
     switch (split) {                                     \
         case 2: GS_ONESWEEP(8, I, 2); break;             \

@@ -105,9 +105,7 @@ void launch_onesweep(uint32_t digit_bits, const uint32_t* keys_in, const uint32_
                      uint32_t* vals_out, const uint32_t* n_dev, uint32_t n_host, uint32_t max_n, uint32_t shift,
                      uint32_t dmask, const uint32_t* hist, FrameCtl* ctl, uint64_t* flags, uint32_t slot,
                      int grid_cap, cudaStream_t s, uint32_t block = kSortPartition, uint32_t split = 0,
-                     bool early = false, uint32_t* ranges = nullptr, uint32_t tiles = 0);
-// early: *n_dev (or n_host), hist, ctl->seq and the ticket counter were written at least two kernels
-// back on the stream, so they are read before the programmatic-launch wait for the previous kernel.
+                     uint32_t* ranges = nullptr, uint32_t tiles = 0);
 // ranges (the last pass of a frame's sort only): each tile's (first, last + 1) in the sorted keys is
 // combined into ranges[2 tile], ranges[2 tile + 1] by atomic min / max over the CTAs; the ranges must
 // hold (0xFFFFFFFF, 0) before the pass (launch_frame_begin) and launch_tile_order, which reads them
