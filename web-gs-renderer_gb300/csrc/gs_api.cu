@@ -290,7 +290,7 @@ int ensure_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a) {
         GS_CK(f.vals[b].reserve(a.max_instance));
     }
     const size_t sort_parts = ((size_t)a.max_instance + ctx->cfg.sort_block - 1) / ctx->cfg.sort_block;
-    const size_t scan_parts = ((size_t)a.n + 1 + kScanPartition - 1) / kScanPartition;
+    const size_t scan_parts = ((size_t)a.n + 1 + kEmitPartitionMin - 1) / kEmitPartitionMin;
     const size_t words = std::max(onesweep_flag_words(sort_parts, radix), scan_parts);
     if (words > f.flags.cap || !f.flags.p) {
         GS_CK(f.flags.reserve(words));

@@ -122,8 +122,9 @@ __global__ void k_frame_begin_multi(MultiViewFrames mv) {
 }
 
 // ---- fused offset scan + emit ---------------------------------------------------------------
-// Partition p covers entries [p*2048, p*2048+2048) of counts[0..n] (n+1 entries; counts[n] = 0).
-// 1. each thread loads 8 consecutive counts (two 16-byte loads), the block scans them;
+// Partition p covers entries [p*PART, p*PART+PART) of counts[0..n] (n+1 entries; counts[n] = 0), PART = 256
+// ITEMS: fewer Gaussians for a smaller scene (the rule is at launch_scan_emit).
+// 1. each thread loads ITEMS consecutive counts, the block scans them;
 // 2. the partition publishes its aggregate and sums its predecessors' aggregates in parallel;
 // 3. offsets[g] are written (offsets[n] = I), the partition holding entry n publishes I and
 //    min(I, max_instance) to FrameCtl (indirect_arg.wgsl:14-27);
@@ -133,6 +134,9 @@ __global__ void k_frame_begin_multi(MultiViewFrames mv) {
 //    order (emit.wgsl:55-66) and slots >= max_instance are dropped (:57-59);
 // 5. the digit histograms of every sort pass are accumulated on the fly (per Gaussian for the
 //    depth digits, per instance for the tile digits).
+constexpr uint32_t kEmitItems = 8;                            // slots per thread of an emit chunk
+constexpr uint32_t kEmitChunk = kEmitItems * kScanThreads;    // slots per emit chunk
+template <uint32_t ITEMS>
 __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __restrict__ counts,
                                                             const uint4* __restrict__ meta, uint32_t n,
                                                             uint32_t tiles_x, uint32_t max_instance,
@@ -140,9 +144,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
                                                             uint32_t* __restrict__ offsets, uint32_t* __restrict__ keys,
                                                             uint32_t* __restrict__ vals, FrameCtl* ctl,
                                                             uint64_t* flags, uint32_t slot) {
-    __shared__ uint32_t s_off[kScanPartition + 1];
-    __shared__ uint2 s_meta[kScanPartition];  // (minX | minY << 16, rect width | depth16 << 16)
-    __shared__ uint32_t s_own[kScanPartition];  // owner (local Gaussian) of each slot of an emit chunk
+    constexpr uint32_t PART = ITEMS * kScanThreads;  // Gaussians per partition
+    __shared__ uint32_t s_off[PART + 1];
+    __shared__ uint2 s_meta[PART];  // (minX | minY << 16, rect width | depth16 << 16)
+    __shared__ uint32_t s_own[kEmitChunk];  // owner (local Gaussian) of each slot of an emit chunk
     __shared__ uint32_t s_hist[8 * 256];
     __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
     __shared__ uint32_t s_part, s_excl, s_seq;
@@ -158,21 +163,28 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
     __syncthreads();
     const uint32_t part = s_part, seq = s_seq;
     const uint32_t entries = n + 1u;
-    const uint32_t base = part * kScanPartition;
-    const uint32_t g0 = base + tid * kScanItems;
+    const uint32_t base = part * PART;
+    const uint32_t g0 = base + tid * ITEMS;
 
-    uint32_t c[kScanItems];
-    if (g0 + kScanItems <= entries) {
-        const uint4 a = *reinterpret_cast<const uint4*>(counts + g0);
-        const uint4 b = *reinterpret_cast<const uint4*>(counts + g0 + 4);
-        c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w; c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
+    uint32_t c[ITEMS];
+    if (g0 + ITEMS <= entries) {
+        if constexpr (ITEMS >= 4u) {
+#pragma unroll
+            for (uint32_t k = 0; k < ITEMS; k += 4u) {
+                const uint4 a = *reinterpret_cast<const uint4*>(counts + g0 + k);
+                c[k] = a.x; c[k + 1u] = a.y; c[k + 2u] = a.z; c[k + 3u] = a.w;
+            }
+        } else {
+#pragma unroll
+            for (uint32_t k = 0; k < ITEMS; ++k) c[k] = counts[g0 + k];
+        }
     } else {
 #pragma unroll
-        for (uint32_t k = 0; k < kScanItems; ++k) c[k] = (g0 + k < entries) ? counts[g0 + k] : 0u;
+        for (uint32_t k = 0; k < ITEMS; ++k) c[k] = (g0 + k < entries) ? counts[g0 + k] : 0u;
     }
     uint32_t tsum = 0, vis = 0;
 #pragma unroll
-    for (uint32_t k = 0; k < kScanItems; ++k) {
+    for (uint32_t k = 0; k < ITEMS; ++k) {
         tsum += c[k];
         vis += c[k] != 0u ? 1u : 0u;
     }
@@ -186,8 +198,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
     {
         uint32_t run = texcl;
 #pragma unroll
-        for (uint32_t k = 0; k < kScanItems; ++k) {
-            const uint32_t lg = tid * kScanItems + k;
+        for (uint32_t k = 0; k < ITEMS; ++k) {
+            const uint32_t lg = tid * ITEMS + k;
             s_off[lg] = run;
             if (c[k] != 0u) {
                 const uint4 m = meta[g0 + k];
@@ -196,7 +208,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
             }
             run += c[k];
         }
-        if (tid == 0) s_off[kScanPartition] = total;
+        if (tid == 0) s_off[PART] = total;
     }
     // sum the aggregates of all predecessors: every partition publishes before it waits on anything
     // and its predecessors hold smaller tickets (they are running or done), so the waits end without
@@ -229,11 +241,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
 
     // offsets (the debug view of offset_scan.wgsl's in-place result)
 #pragma unroll
-    for (uint32_t k = 0; k < kScanItems; ++k) {
+    for (uint32_t k = 0; k < ITEMS; ++k) {
         const uint32_t g = g0 + k;
-        if (g < entries) offsets[g] = excl + s_off[tid * kScanItems + k];
+        if (g < entries) offsets[g] = excl + s_off[tid * ITEMS + k];
         if (g == n) {
-            const uint32_t I = excl + s_off[tid * kScanItems + k];
+            const uint32_t I = excl + s_off[tid * ITEMS + k];
             ctl->instance_count = I;
             ctl->sorted_count = I < max_instance ? I : max_instance;
             if (I > max_instance) atomicOr(&ctl->status, kDevOverflow);
@@ -245,8 +257,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
     const uint32_t mask = radix - 1u;
     const uint32_t depth_passes = min(passes, 16u / digit_bits);
 #pragma unroll
-    for (uint32_t k = 0; k < kScanItems; ++k) {
-        const uint32_t lg = tid * kScanItems + k;
+    for (uint32_t k = 0; k < ITEMS; ++k) {
+        const uint32_t lg = tid * ITEMS + k;
         if (c[k] == 0u) continue;
         const uint32_t first = excl + s_off[lg];
         const uint32_t kept = first >= max_instance ? 0u : min(c[k], max_instance - first);
@@ -256,20 +268,20 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
             atomicAdd(&s_hist[p * radix + ((d16 >> (p * digit_bits)) & mask)], kept);
     }
 
-    // emit, in chunks of kScanPartition slots: the owner of every slot of a chunk comes from an owner
+    // emit, in chunks of kEmitChunk slots: the owner of every slot of a chunk comes from an owner
     // map (each Gaussian marks the slot where its run starts, or slot 0 if its run covers the chunk's
     // start; an inclusive max-scan fills the rest, local indices growing with their offsets), so no
     // slot searches; the tile of instance k of a w-wide rect is (k / w, k % w) through a float
     // reciprocal corrected to the exact quotient
     const uint32_t kept_total = excl >= max_instance ? 0u : min(total, max_instance - excl);
-    for (uint32_t c0 = 0; c0 < kept_total; c0 += kScanPartition) {
-        const uint32_t c1 = c0 + kScanPartition;
+    for (uint32_t c0 = 0; c0 < kept_total; c0 += kEmitChunk) {
+        const uint32_t c1 = c0 + kEmitChunk;
 #pragma unroll
-        for (uint32_t k = 0; k < kScanItems; ++k) s_own[tid * kScanItems + k] = 0u;
+        for (uint32_t k = 0; k < kEmitItems; ++k) s_own[tid * kEmitItems + k] = 0u;
         __syncthreads();
 #pragma unroll
-        for (uint32_t k = 0; k < kScanItems; ++k) {
-            const uint32_t lg = tid * kScanItems + k;
+        for (uint32_t k = 0; k < ITEMS; ++k) {
+            const uint32_t lg = tid * ITEMS + k;
             if (c[k] == 0u) continue;
             const uint32_t start = s_off[lg];
             if (start >= c0 && start < c1) s_own[start - c0] = lg;
@@ -278,16 +290,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
         __syncthreads();
         uint32_t run = 0;
 #pragma unroll
-        for (uint32_t k = 0; k < kScanItems; ++k) run = max(run, s_own[tid * kScanItems + k]);
+        for (uint32_t k = 0; k < kEmitItems; ++k) run = max(run, s_own[tid * kEmitItems + k]);
         const uint32_t before = block_exclusive_max<kScanThreads>(run, s_warp);
         run = before;
 #pragma unroll
-        for (uint32_t k = 0; k < kScanItems; ++k) {
-            run = max(run, s_own[tid * kScanItems + k]);
-            s_own[tid * kScanItems + k] = run;
+        for (uint32_t k = 0; k < kEmitItems; ++k) {
+            run = max(run, s_own[tid * kEmitItems + k]);
+            s_own[tid * kEmitItems + k] = run;
         }
         __syncthreads();
-        const uint32_t cn = min(kept_total - c0, kScanPartition);
+        const uint32_t cn = min(kept_total - c0, kEmitChunk);
         for (uint32_t j = tid; j < cn; j += kScanThreads) {
             const uint32_t i = c0 + j;
             const uint32_t lg = s_own[j];
@@ -746,9 +758,21 @@ void launch_frame_begin(FrameCtl* ctl, uint64_t* flags, uint32_t flag_words, cud
 void launch_scan_emit(const uint32_t* counts, const uint4* meta, uint32_t n, uint32_t tiles_x, uint32_t max_instance,
                       uint32_t digit_bits, uint32_t passes, uint32_t* offsets, uint32_t* keys, uint32_t* vals,
                       FrameCtl* ctl, uint64_t* flags, uint32_t slot, cudaStream_t s) {
-    const uint32_t parts = (n + 1u + kScanPartition - 1u) / kScanPartition;
-    launch_pdl(k_scan_emit, dim3(parts), dim3(kScanThreads), s, counts, meta, n, tiles_x, max_instance, digit_bits,
-               passes, offsets, keys, vals, ctl, flags, slot);
+    auto launch = [&](auto kernel, uint32_t items) {
+        const uint32_t part = items * kScanThreads, parts = (uint32_t)(((uint64_t)n + part) / part);  // n + 1 entries
+        launch_pdl(kernel, dim3(parts), dim3(kScanThreads), s, counts, meta, n, tiles_x, max_instance, digit_bits, passes,
+                   offsets, keys, vals, ctl, flags, slot);
+    };
+    // The emit of a partition is one CTA's work, so a small scene needs small partitions to fill the GPU (a
+    // close-up's Gaussians emit dozens of instances each), while the predecessor sums and the histograms' global
+    // adds cost per partition. Measured in us with 256 / 512 / 1024 / 2048 Gaussians per partition: 50k at
+    // 512x512 13.8 / 13.2 / 15.7 / 28.5, a close-up of 60k 27.8 / 37.6 / 54 / 99, 100k at 320x240 14.5 / 13.6 /
+    // 12.3 / 19.0, 250k in 8x8 tiles 31 / 26 / 24.7 / 32.4, 500k 44 / 30 / 17.8 / 19.8, 1M 80 / 49 / 28.9 / 30.8,
+    // 3M at 4K - / - / 97 / 113, 8M - / - / 171 / 164, 16M - / - / 365 / 344
+    if (n < 75000u) launch(k_scan_emit<1>, 1u);
+    else if (n < 150000u) launch(k_scan_emit<2>, 2u);
+    else if (n < 8000000u) launch(k_scan_emit<4>, 4u);
+    else launch(k_scan_emit<8>, 8u);
 }
 
 void launch_exclusive_scan(uint32_t* data, uint32_t n, uint32_t* total_dev, FrameCtl* ctl, uint64_t* flags,

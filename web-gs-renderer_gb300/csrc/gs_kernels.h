@@ -80,6 +80,7 @@ void launch_preprocess(const float* rows, uint32_t stride, uint32_t n, const Vie
 constexpr uint32_t kScanItems = 8;
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanPartition = kScanItems * kScanThreads;
+constexpr uint32_t kEmitPartitionMin = kScanThreads;  // smallest partition of launch_scan_emit
 void launch_scan_emit(const uint32_t* counts, const uint4* meta, uint32_t n, uint32_t tiles_x, uint32_t max_instance,
                       uint32_t digit_bits, uint32_t passes, uint32_t* offsets, uint32_t* keys, uint32_t* vals,
                       FrameCtl* ctl, uint64_t* flags, uint32_t slot, cudaStream_t s);
