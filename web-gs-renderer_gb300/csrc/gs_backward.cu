@@ -5,7 +5,8 @@
 //                         recomputing power and alpha bit for bit as the forward did (same pinned
 //                         arithmetic), recovering T by division, and accumulating dL/d(pixel.xy, conic,
 //                         opacity, colour) per Gaussian: eight hits at a time reduced over the block's
-//                         pixels by matrix instructions, three vector atomics per hit.
+//                         pixels by matrix instructions, three vector atomics per hit. Up to the pixel's own
+//                         chain the arithmetic runs on two hits at once by packed fp32 operations.
 // The preprocess half (2D gradients -> the 59 attributes) is in gs_preprocess_backward.cu.
 // Conventions: gradients flow through the fp32 RGB before quantization; culled Gaussians, skipped
 // pairs and splats after a pixel's termination get none; active clamps (alpha 0.99, colour >= 0)
@@ -116,6 +117,35 @@ __device__ __forceinline__ void pix_step(PixState& p, uint32_t pos, const float4
     p.d = __fmaf_rn(w, k, p.d);
 }
 
+// The same for two splats, the one at the higher position first (back to front): what does not depend on the
+// pixel's state is formed for both at once by packed operations (each half rounds like the scalar form).
+// Pairs as the walk lays them out; opacity 0 stands for one below every cut-off (its alpha is 0).
+__device__ __forceinline__ void pix_step2(PixState& p, const float4& p0, const float4& p1, const float4& p2,
+                                          const float4& p3, const float4& p4, float2& gp, float2& w) {
+    const float2 dx = __fadd2_rn(make_float2(p0.x, p0.y), both(-p.fx)), dy = __fadd2_rn(make_float2(p0.z, p0.w), both(-p.fy));
+    const float2 q = __ffma2_rn(__fmul2_rn(make_float2(p1.x, p1.y), dx), dx,
+                                __fmul2_rn(__fmul2_rn(make_float2(p2.x, p2.y), dy), dy));
+    const float2 power = __ffma2_rn(both(-0.5f), q, __fmul2_rn(__fmul2_rn(make_float2(p1.z, p1.w), dx), dy));
+    const float2 og = raster_alpha_unclamped2(make_float2(p2.z, p2.w),
+                                              make_float2(max_nan(power.x, kPowerFloor), max_nan(power.y, kPowerFloor)));
+    const float2 kk = __ffma2_rn(make_float2(p3.x, p3.y), both(p.dr),
+                                 __ffma2_rn(make_float2(p3.z, p3.w), both(p.dg), __fmul2_rn(make_float2(p4.x, p4.y), both(p.db))));
+    auto one = [&](float power, float og, float k, uint32_t pos, float& gp, float& w) {
+        float alpha = fminf(kAlphaClamp, og);
+        const bool in = (pos <= p.L) & !(power > 0.0f) & (alpha >= kEpsilon);
+        alpha = in ? alpha : 0.0f;
+        k = in ? k : 0.0f;
+        const float ria = fast_rcp(1.0f - alpha);
+        p.T = p.T * ria;
+        w = alpha * p.T;
+        const float dalpha = __fmaf_rn(p.T, k, -(p.d * ria));
+        gp = og <= kAlphaClamp ? dalpha * alpha : 0.0f;
+        p.d = __fmaf_rn(w, k, p.d);
+    };
+    one(power.x, og.x, kk.x, __float_as_uint(p4.z), gp.x, w.x);
+    one(power.y, og.y, kk.y, __float_as_uint(p4.w), gp.y, w.y);
+}
+
 __device__ __forceinline__ bool pix_finite(const PixState& p) {
     return finite_f(p.dr) && finite_f(p.dg) && finite_f(p.db);
 }
@@ -149,7 +179,8 @@ __device__ __noinline__ void walk_alone(PixState p, const uint32_t* __restrict__
 
 constexpr uint32_t kRowUnits = 20;  // 16-byte units per row: 16 pixel pairs, padded so that the eight
                                     // lanes that read two rows at once hit distinct banks
-constexpr uint32_t kRing = 64;      // staged hits per warp (a multiple of kHits, at least 32 + 31)
+constexpr uint32_t kRing = 64;      // staged hits per warp (room for 32 more at two flushes' pending)
+constexpr uint32_t kChunk = 32;     // most hits laid out in pairs at once
 constexpr uint32_t kBwdWarps = 2;   // warps per CTA; they share nothing
 
 // Shared memory of a warp: a ring of staged hits and the rows of kHits of them. A unit of a row holds two
@@ -158,6 +189,8 @@ struct BwdWarp {
     float4 a[kRing];  // (x, y, conic.x, conic.y)
     float4 b[kRing];  // (conic.z, opacity, r, g)
     float4 c[kRing];  // (b, cut, range position, Gaussian)
+    float4 pair[kChunk / 2][5];  // (x, x', y, y'), (A, A', -B, -B'), (C, C', o, o'), (r, r', g, g'),
+                                 // (b, b', position, position')
     float4 rows[kHits * kRowUnits];
 };
 
@@ -169,13 +202,14 @@ struct BwdWarp {
 // batches, computed the cull again and met at two barriers per batch, a hit's bookkeeping (finding the
 // next bit, addresses, the counter of the pending rows) is gone.
 //
-// Bound by instruction issue (77% of slots at 28 warps per SM) where the blocks fill the GPU, by the
-// longest list otherwise. Measured against the CTA per tile with shuffle reductions and two pixels per
-// lane, mixture scenes: 1M / 1080p 427M -> 276M warp instructions, 839k -> 603k cycles; 3M / 1080p
-// 879 -> 640 us; 500k / 720p (a list of 2300 splats) 358 -> 150 us; 20k / 397x301 92 -> 30 us. On the way,
-// 1M / 1080p: matrix sums but a CTA per tile, 8x8 blocks with two pixels per lane 1008k cycles, 8x4 blocks
-// 847k; 8x4 blocks by the hit masks 693k; the chain's divide as one reciprocal and no branch in a hit
-// 664k; columns without selects and predicated atomics 631k; heads by integer rounding 603k.
+// Bound by instruction issue (73% of slots at 28 warps per SM) and shared-memory reads (67%) where the
+// blocks fill the GPU, by the longest list otherwise. Measured against a CTA per tile with shuffle
+// reductions and two pixels per lane, mixture scenes: 1M / 1080p 405 -> 284 us (427M -> 250M warp
+// instructions); 3M / 1080p 879 -> 584; 500k / 720p (a list of 2300 splats) 358 -> 141; 20k / 397x301 92 -> 24. On
+// the way, 1M / 1080p in thousand cycles, from 839: matrix sums but a CTA per tile, 8x8 blocks with two pixels
+// per lane 1008, 8x4 blocks 847; 8x4 blocks by the hit masks 693; the chain's divide as one reciprocal and no
+// branch in a hit 664; columns without selects and predicated atomics 631; heads by integer rounding 603;
+// hits in pairs on packed operations 577, their loop fully unrolled 560.
 template <int TILE>
 __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backward(const uint32_t* __restrict__ ranges,
                                                                      const uint32_t* __restrict__ vals,
@@ -249,14 +283,32 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
     }
     const float cx = (float)bx0 + kCx, cy = (float)by0 + kCy;
 
-    // visits the eight staged hits from ring slot h0 on and adds the gradients of the first cnt of them
-    auto visit = [&](uint32_t h0, uint32_t cnt) {
+    // lays the next cnt (at most kChunk) staged hits out as pairs, a lane each
+    auto lay_out = [&](uint32_t h0, uint32_t cnt) {
+        const uint32_t slot = (h0 + lane) % kRing;
+        float4 a = sh.a[slot], b = sh.b[slot], c = sh.c[slot];
+        float* q = reinterpret_cast<float*>(sh.pair[lane >> 1]) + (lane & 1u);
+        if (c.y > 0.0f) b.y = 0.0f;  // a positive cut-off: the opacity itself is below 1/255
+        if (lane >= cnt) {           // past the hits: a position no pixel blends
+            a = b = c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            c.z = __uint_as_float(0xFFFFFFFFu);
+        }
+        q[0] = a.x; q[2] = a.y; q[4] = a.z; q[6] = -a.w;
+        q[8] = b.x; q[10] = b.y; q[12] = b.z; q[14] = b.w;
+        q[16] = c.x; q[18] = c.z;
+        __syncwarp();
+    };
+    // visits hits 8 v to 8 v + 7 of those laid out, which are staged from ring slot h0 on, and adds the
+    // gradients of the first cnt of them
+    auto visit = [&](uint32_t v, uint32_t h0, uint32_t cnt) {
 #pragma unroll
-        for (uint32_t u = 0; u < kHits; ++u) {
-            const float4 c = sh.c[h0 + u];
-            float gp, w;
-            pix_step(p, __float_as_uint(c.z), sh.a[h0 + u], sh.b[h0 + u], make_float2(c.x, c.y), gp, w);
-            reinterpret_cast<float2*>(sh.rows)[2u * kRowUnits * u + lane] = make_float2(gp, w);
+        for (uint32_t u = 0; u < kHits / 2u; ++u) {
+            const float4* r = sh.pair[4u * v + u];
+            float2 gp, w;
+            pix_step2(p, r[0], r[1], r[2], r[3], r[4], gp, w);
+            float2* row = reinterpret_cast<float2*>(sh.rows) + 4u * kRowUnits * u + lane;
+            row[0] = make_float2(gp.x, w.x);
+            row[2u * kRowUnits] = make_float2(gp.y, w.y);
         }
         __syncwarp();
         float m[4] = {0.0f, 0.0f, 0.0f, 0.0f}, q[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -276,9 +328,10 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
         const float suv = __shfl_sync(0xffffffffu, m[0], 2, 4), svv = __shfl_sync(0xffffffffu, m[1], 2, 4);
         const float c0 = q[2] + __shfl_xor_sync(0xffffffffu, q[2], 2);  // r (fc 0), b (fc 1)
         const float c1 = q[3] + __shfl_xor_sync(0xffffffffu, q[3], 2);  // g (fc 0)
-        const float4 a = sh.a[h0 + fr];
-        const float2 b = *reinterpret_cast<const float2*>(&sh.b[h0 + fr]);
-        const uint32_t gi = __float_as_uint(sh.c[h0 + fr].w);
+        const uint32_t slot = (h0 + fr) % kRing;
+        const float4 a = sh.a[slot];
+        const float2 b = *reinterpret_cast<const float2*>(&sh.b[slot]);
+        const uint32_t gi = __float_as_uint(sh.c[slot].w);
         const float X = a.x - cx, Y = a.y - cy;
         const float sx = __fmaf_rn(X, s0, -su), sy = __fmaf_rn(Y, s0, -sv);  // sums of gp dx, gp dy
         const float sxx = __fmaf_rn(X, sx - su, suu), syy = __fmaf_rn(Y, sy - sv, svv);
@@ -314,9 +367,14 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
     };
 
     uint32_t head = 0, ready = 0, tail = 0;  // hits visited, staged for certain, staged or on their way
+    auto process = [&](uint32_t cnt) {
+        lay_out(head, cnt);
+        for (uint32_t v = 0; kHits * v < cnt; ++v) visit(v, head + kHits * v, min(kHits, cnt - kHits * v));
+        head += cnt;
+    };
     next_group();
     while (true) {
-        while (m != 0u && tail - head <= kRing - 32u) {
+        while (m != 0u && tail - head + __popc(m) <= kRing) {
             if (m >> lane & 1u) {
                 const uint32_t slot = (tail + __popc(m >> lane) - 1u) % kRing;  // back to front
                 const bool ok = gnext < n;
@@ -335,12 +393,12 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
         if (m == 0u) break;
         cp_async_wait<1>();
         __syncwarp();
-        for (uint32_t k = 0; k < 2u && ready - head >= kHits; ++k, head += kHits) visit(head % kRing, kHits);
+        if (ready - head >= 2u * kHits) process(min(kChunk, ready - head) & ~(kHits - 1u));
         ready = tail;
     }
     cp_async_wait<0>();
     __syncwarp();
-    for (; head < tail; head += kHits) visit(head % kRing, min(kHits, tail - head));
+    while (head < tail) process(min(kChunk, tail - head));
 }
 
 template <int TILE, typename... Args>

@@ -85,15 +85,6 @@ struct RasterShared {
     uint32_t masks[kMaxGroups][kWarps];  // the step's hits per group and warp
 };
 
-// max that keeps a NaN. Below the floor no splat of any opacity reaches 1/255, and from it up o * exp(power)
-// stays normal for an opacity of at least 1/255.
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float m;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
-    return m;
-}
-constexpr float kPowerFloor = -20.0f;
-
 // What a raster keeps besides the colours: nothing, the final transmittance, or that and the contributor
 // count (and, for a differentiable frame, the hit masks).
 constexpr int kKeepNothing = 0, kKeepT = 1, kKeepLast = 2;

@@ -84,6 +84,15 @@ __device__ __forceinline__ float2 raster_alpha_unclamped2(float2 o, float2 x) {
                        __int_as_float(__float_as_int(op.y) + (__float_as_int(t.y) << 23)));
 }
 
+// max that keeps a NaN. Below the floor no splat of any opacity reaches 1/255, and from it up o * exp(power)
+// stays normal for an opacity of at least 1/255.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+constexpr float kPowerFloor = -20.0f;
+
 __device__ __forceinline__ bool finite_f(float v) { return fabsf(v) <= 3.0e38f; }
 
 // Half extents of a splat's octagon along x, y, u = x + y and v = x - y, for pixels within `reach` of its
