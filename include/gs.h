@@ -174,7 +174,8 @@ typedef struct gs_batch_view {
 
 /* Batched forward (no counterpart in the reference, which renders one view per execute()): all
  * views, of any scenes and resolutions, are captured into one CUDA graph and forked over the
- * context's side streams, so small views share the GPU. Every view's output must use the same
+ * context's side streams, so small views share the GPU (many small views of one scene share every
+ * launch too). Every view's output must use the same
  * location. Same results as gs_forward per view. */
 int gs_forward_batch(gs_ctx* ctx, const gs_batch_view* views, uint32_t count);
 

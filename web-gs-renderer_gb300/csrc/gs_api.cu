@@ -161,8 +161,7 @@ struct gs_ctx {
     gs_config cfg{};
     cudaStream_t stream = nullptr;
     cudaStream_t side[kSideStreams] = {};
-    cudaEvent_t fork = nullptr, join[kSideStreams] = {};
-    cudaEvent_t group_done[kSideStreams] = {};  // a batch's per-scene preprocess, one per group
+    cudaEvent_t fork = nullptr, views_ready = nullptr, join[kSideStreams] = {};
     std::string err;
 
     Frame main;                  // gs_forward / gs_backward
@@ -354,42 +353,64 @@ RasterOut raster_out(const gs_ctx* ctx, Frame& f, const gs_image* out, size_t ma
     return ro;
 }
 
-// Enqueues one frame (renderer.js:822-932) on stream s; preprocessed: its frame control block was
-// reset and its preprocess done already (by a multi-view preprocess of its scene).
-void enqueue_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a, cudaStream_t s, bool profile, bool preprocessed = false) {
+// Enqueues the passes after the preprocess (renderer.js:836-932) of `count` frames (1 to kMaxRunViews) on stream s,
+// every stage one launch for all of them. profile: events around the stages, from kPassScanEmit on.
+void enqueue_views(gs_ctx* ctx, Frame* const* frames, const FrameArgs* args, uint32_t count, cudaStream_t s, bool profile) {
     const uint32_t bits = ctx->cfg.digit_bits, radix = 1u << bits;
-    FrameCtl* ctl = f.ctl.p;
-    if (profile) cudaEventRecord(ctx->ev[0], s);
-    if (!preprocessed) launch_frame_begin(ctl, f.flags.p, (uint32_t)f.flags.cap, s, f.ranges.p, a.tiles_x * a.tiles_y * 2u);
-    if (profile) cudaEventRecord(ctx->ev[1], s);
-    if (!preprocessed) {
-        launch_preprocess(a.scene->rows, a.scene->stride, a.n, a.view, ctx->cfg.tile_size, f.rec.p, f.meta.p,
-                          f.counts.p, ctl, s);
+    EmitView emit[kMaxRunViews];
+    OrderView order[kMaxRunViews];
+    RasterView raster[kMaxRunViews];
+    uint32_t passes = 0, key_bits = 0;
+    for (uint32_t v = 0; v < count; ++v) {
+        Frame& f = *frames[v];
+        const FrameArgs& a = args[v];
+        const uint32_t tiles = a.tiles_x * a.tiles_y, sorted = a.passes & 1u;
+        emit[v] = EmitView{f.counts.p, f.meta.p, f.offsets.p, f.keys[0].p, f.vals[0].p, f.ctl.p, f.flags.p,
+                           a.n, a.tiles_x, a.max_instance, a.passes};
+        order[v] = OrderView{f.ranges.p, f.order_hist.p, f.order.p, &f.ctl.p->status, tiles};
+        raster[v] = RasterView{f.ranges.p, f.vals[sorted].p, f.rec.p, f.ctl.p, f.order.p, a.out, a.n, a.w, a.h, a.tiles_x, tiles};
+        passes = std::max(passes, a.passes);
+        key_bits = std::max(key_bits, 16u + bitlen(tiles - 1u));
     }
-    if (profile) cudaEventRecord(ctx->ev[2], s);
-    launch_scan_emit(f.counts.p, f.meta.p, a.n, a.tiles_x, a.max_instance, bits, a.passes, f.offsets.p, f.keys[0].p,
-                     f.vals[0].p, ctl, f.flags.p, 0, s);
-    if (profile) cudaEventRecord(ctx->ev[3], s);
-    int cur = 0;
-    const uint32_t key_bits = 16u + bitlen(a.tiles_x * a.tiles_y - 1u);
-    for (uint32_t p = 0; p < a.passes; ++p) {
+    launch_scan_emit(emit, count, bits, 0, s);
+    if (profile) cudaEventRecord(ctx->ev[kPassScanEmit + 1], s);
+    for (uint32_t p = 0; p < passes; ++p) {
         // the tile digits arrive in depth order, nearly all distinct within a warp: their ranking
         // matches the high half of the digit and separates the low half by ballots (w/2 of a w-bit
         // digit, from 2 bits up); the depth digits keep the plain match
         const uint32_t w = std::min(bits, key_bits - p * bits);
         const uint32_t split = p * bits >= 16u && w / 2u >= 2u ? w / 2u : 0u;
-        launch_onesweep(bits, f.keys[cur].p, f.vals[cur].p, f.keys[cur ^ 1].p, f.vals[cur ^ 1].p, &ctl->sorted_count,
-                        0, a.max_instance, p * bits, radix - 1u, ctl->hist + p * radix, ctl, f.flags.p, 1 + p, 0, s,
-                        ctx->cfg.sort_block, split,
-                        p + 1 == a.passes ? f.ranges.p : nullptr, a.tiles_x * a.tiles_y);  // the last pass: ranges
-        cur ^= 1;
+        SortView sort[kMaxRunViews];
+        uint32_t k = 0;
+        for (uint32_t v = 0; v < count; ++v) {
+            Frame& f = *frames[v];
+            const FrameArgs& a = args[v];
+            if (p >= a.passes) continue;  // a smaller image may need fewer passes
+            const uint32_t cur = p & 1u;
+            sort[k++] = SortView{f.keys[cur].p, f.vals[cur].p, f.keys[cur ^ 1].p, f.vals[cur ^ 1].p, &f.ctl.p->sorted_count,
+                                 f.ctl.p->hist + p * radix, f.ctl.p, f.flags.p,
+                                 p + 1 == a.passes ? f.ranges.p : nullptr,  // the last pass: ranges
+                                 0, a.max_instance, radix - 1u, a.tiles_x * a.tiles_y};
+        }
+        launch_onesweep(sort, k, bits, p * bits, 1 + p, s, ctx->cfg.sort_block, split);
     }
-    if (profile) cudaEventRecord(ctx->ev[4], s);
-    launch_tile_order(f.ranges.p, a.tiles_x * a.tiles_y, f.order_hist.p, f.order.p, &ctl->status, s);
-    if (profile) cudaEventRecord(ctx->ev[5], s);
-    launch_raster(ctx->cfg.tile_size, ctx->cfg.raster_batch, f.ranges.p, f.vals[cur].p, f.rec.p, a.n, ctl, a.w, a.h,
-                  a.tiles_x, a.tiles_y, a.out, f.order.p, s);
-    if (profile) cudaEventRecord(ctx->ev[6], s);
+    if (profile) cudaEventRecord(ctx->ev[kPassSort + 1], s);
+    launch_tile_order(order, count, s);
+    if (profile) cudaEventRecord(ctx->ev[kPassRanges + 1], s);
+    launch_raster(raster, count, ctx->cfg.tile_size, ctx->cfg.raster_batch, s);
+    if (profile) cudaEventRecord(ctx->ev[kPassRaster + 1], s);
+}
+
+// Enqueues one frame (renderer.js:822-932) on stream s.
+void enqueue_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a, cudaStream_t s, bool profile) {
+    if (profile) cudaEventRecord(ctx->ev[kPassBegin], s);
+    launch_frame_begin(f.ctl.p, f.flags.p, (uint32_t)f.flags.cap, s, f.ranges.p, a.tiles_x * a.tiles_y * 2u);
+    if (profile) cudaEventRecord(ctx->ev[kPassBegin + 1], s);
+    launch_preprocess(a.scene->rows, a.scene->stride, a.n, a.view, ctx->cfg.tile_size, f.rec.p, f.meta.p, f.counts.p,
+                      f.ctl.p, s);
+    if (profile) cudaEventRecord(ctx->ev[kPassPreprocess + 1], s);
+    Frame* const one = &f;
+    enqueue_views(ctx, &one, &a, 1, s, profile);
 }
 
 void remember(Frame& f, const FrameArgs& a) {
@@ -433,6 +454,17 @@ struct CameraPrologue {
     uint32_t count = 0;
 };
 
+// Views that share one launch per stage, of `count` views of one scene in a batch; work: the largest
+// view's Gaussians + pixels. A launch costs about 1.3 us of a graph whatever it does, which is all that
+// a turntable of thumbnails spends: 24 views of 2k Gaussians at 64x64 take 248 us forked one by one and
+// 176 us in runs of 8, of 100k at 320x240 921 and 850, 16 of 200k at 640x480 1683 and 1586. Few views
+// fill a run badly and lose the overlap of one view's sort with another's raster (4 views of 100k, three
+// such batches side by side: 137 and 144 us each), and so do full-screen ones, whose launches cost
+// nothing beside their work (16 views of 15k at 1080p: 370 and 417 us; of 500k: 1203 and 1214).
+uint32_t views_per_run(uint32_t count, uint64_t work) {
+    return count >= kMaxRunViews && work < 1000000u ? kMaxRunViews : 1u;
+}
+
 int capture_and_launch(gs_ctx* ctx, cudaGraphExec_t* exec, GraphKey* cached, const GraphKey& key,
                        const std::vector<Frame*>& frames, const std::vector<FrameArgs>& args,
                        const CameraPrologue& prologue = CameraPrologue{}) {
@@ -445,51 +477,53 @@ int capture_and_launch(gs_ctx* ctx, cudaGraphExec_t* exec, GraphKey* cached, con
         if (frames.size() == 1) {
             enqueue_frame(ctx, *frames[0], args[0], ctx->stream, false);
         } else {
-            // views are independent: fork them over the side streams so small views fill the GPU
-            // together. Views of one scene are preprocessed together (one pass over the scene's
-            // attributes per group of up to 16 views) on the stream of the group's first view, so the
-            // groups' preprocesses run side by side; a view on another stream waits for its group.
+            // the views of one scene take one pass over its attributes, up to 16 views at a time, and then fork
+            // over the side streams in runs that share a launch per stage; a scene's only view goes by itself
             cudaEventRecord(ctx->fork, ctx->stream);
             const int used = (int)std::min<size_t>(frames.size(), kSideStreams);
             for (int s = 0; s < used; ++s) cudaStreamWaitEvent(ctx->side[s], ctx->fork, 0);
-            std::vector<int> group_of(frames.size(), -1);
-            int groups = 0;
-            for (size_t i = 0; i < frames.size() && groups < kSideStreams; ++i) {
-                if (group_of[i] >= 0) continue;
-                std::vector<size_t> members;
-                for (size_t j = i; j < frames.size(); ++j)
-                    if (group_of[j] < 0 && args[j].scene == args[i].scene) members.push_back(j);
-                if (members.size() < 2) continue;
-                for (size_t c0 = 0; c0 < members.size() && groups < kSideStreams; c0 += kMaxMultiViews) {
-                    MultiViewFrames mv{};
-                    mv.count = (uint32_t)std::min<size_t>(kMaxMultiViews, members.size() - c0);
-                    for (uint32_t v = 0; v < mv.count; ++v) {
-                        const size_t j = members[c0 + v];
-                        Frame& f = *frames[j];
-                        mv.view[v] = args[j].view;
-                        mv.rec[v] = f.rec.p;
-                        mv.meta[v] = f.meta.p;
-                        mv.counts[v] = f.counts.p;
-                        mv.ctl[v] = f.ctl.p;
-                        mv.ranges[v] = f.ranges.p;
-                        mv.range_words[v] = args[j].tiles_x * args[j].tiles_y * 2u;
-                        mv.flags[v] = f.flags.p;
-                        mv.flag_words[v] = (uint32_t)f.flags.cap;
-                        group_of[j] = groups;
-                    }
-                    cudaStream_t gs = ctx->side[members[c0] % used];
-                    launch_frame_begin_multi(mv, gs);
-                    launch_preprocess_multi(args[i].scene->rows, args[i].scene->stride, args[i].n,
-                                            ctx->cfg.tile_size, mv, gs);
-                    cudaEventRecord(ctx->group_done[groups], gs);
-                    ++groups;
-                }
-            }
+            std::vector<bool> done(frames.size(), false);
+            int next = 0;  // side streams in turn
             for (size_t i = 0; i < frames.size(); ++i) {
-                cudaStream_t s = ctx->side[i % used];
-                const int g = group_of[i];
-                if (g >= 0) cudaStreamWaitEvent(s, ctx->group_done[g], 0);
-                enqueue_frame(ctx, *frames[i], args[i], s, false, g >= 0);
+                if (done[i]) continue;
+                cudaStream_t s = ctx->side[next++ % used];
+                uint64_t work = 0;
+                Frame* group[kMaxMultiViews];
+                FrameArgs group_args[kMaxMultiViews];
+                MultiViewFrames mv{};
+                for (size_t j = i; j < frames.size() && mv.count < kMaxMultiViews; ++j) {
+                    if (done[j] || args[j].scene != args[i].scene) continue;
+                    const uint32_t v = mv.count++;
+                    Frame& f = *frames[j];
+                    done[j] = true;
+                    work = std::max(work, (uint64_t)args[j].n + (uint64_t)args[j].w * args[j].h);
+                    group[v] = &f;
+                    group_args[v] = args[j];
+                    mv.view[v] = args[j].view;
+                    mv.rec[v] = f.rec.p;
+                    mv.meta[v] = f.meta.p;
+                    mv.counts[v] = f.counts.p;
+                    mv.ctl[v] = f.ctl.p;
+                    mv.ranges[v] = f.ranges.p;
+                    mv.range_words[v] = args[j].tiles_x * args[j].tiles_y * 2u;
+                    mv.flags[v] = f.flags.p;
+                    mv.flag_words[v] = (uint32_t)f.flags.cap;
+                }
+                if (mv.count == 1) {
+                    enqueue_frame(ctx, *frames[i], args[i], s, false);
+                    continue;
+                }
+                launch_frame_begin_multi(mv, s);
+                launch_preprocess_multi(args[i].scene->rows, args[i].scene->stride, args[i].n, ctx->cfg.tile_size, mv, s);
+                const uint32_t run = views_per_run(mv.count, work);
+                if (run < mv.count) cudaEventRecord(ctx->views_ready, s);
+                for (uint32_t v = 0; v < mv.count; v += run) {
+                    if (v) {
+                        s = ctx->side[next++ % used];
+                        cudaStreamWaitEvent(s, ctx->views_ready, 0);
+                    }
+                    enqueue_views(ctx, group + v, group_args + v, std::min(run, mv.count - v), s, false);
+                }
             }
             for (int s = 0; s < used; ++s) {
                 cudaEventRecord(ctx->join[s], ctx->side[s]);
@@ -564,9 +598,9 @@ int gs_ctx_create(const gs_config* cfg, gs_ctx** out) {
     bool ok = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) == cudaSuccess;
     for (int s = 0; ok && s < kSideStreams; ++s)
         ok = cudaStreamCreateWithFlags(&ctx->side[s], cudaStreamNonBlocking) == cudaSuccess &&
-             cudaEventCreateWithFlags(&ctx->join[s], cudaEventDisableTiming) == cudaSuccess &&
-             cudaEventCreateWithFlags(&ctx->group_done[s], cudaEventDisableTiming) == cudaSuccess;
+             cudaEventCreateWithFlags(&ctx->join[s], cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming) == cudaSuccess &&
+         cudaEventCreateWithFlags(&ctx->views_ready, cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&ctx->bviews_done, cudaEventDisableTiming) == cudaSuccess &&
          ctx->main.init(ctx->stream) == cudaSuccess && ctx->aux_ctl.reserve(1) == cudaSuccess &&
          cudaMallocHost(&ctx->h_aux, sizeof(FrameCtl)) == cudaSuccess &&
@@ -602,9 +636,9 @@ int gs_ctx_destroy(gs_ctx* ctx) {
     for (int s = 0; s < kSideStreams; ++s) {
         if (ctx->side[s]) cudaStreamDestroy(ctx->side[s]);
         if (ctx->join[s]) cudaEventDestroy(ctx->join[s]);
-        if (ctx->group_done[s]) cudaEventDestroy(ctx->group_done[s]);
     }
     if (ctx->fork) cudaEventDestroy(ctx->fork);
+    if (ctx->views_ready) cudaEventDestroy(ctx->views_ready);
     if (ctx->bviews_done) cudaEventDestroy(ctx->bviews_done);
     if (ctx->h_views) cudaFreeHost(ctx->h_views);
     if (ctx->h_bviews) cudaFreeHost(ctx->h_bviews);
@@ -1325,8 +1359,9 @@ int gs_sort_pairs(gs_ctx* ctx, uint32_t* keys, uint32_t* vals, uint32_t n, uint3
     for (uint32_t p = 0; p < passes; ++p) {
         const uint32_t left = key_bits - p * bits;
         const uint32_t dmask = left >= bits ? radix - 1u : (1u << left) - 1u;
-        launch_onesweep(bits, kb[cur], vb[cur], kb[cur ^ 1], vb[cur ^ 1], nullptr, n, n, p * bits, dmask,
-                        ctl->hist + p * radix, ctl, ctx->aux_flags.p, 1 + p, 0, ctx->stream, ctx->cfg.sort_block);
+        const SortView one{kb[cur], vb[cur], kb[cur ^ 1], vb[cur ^ 1], nullptr, ctl->hist + p * radix, ctl, ctx->aux_flags.p,
+                           nullptr, n, n, dmask, 0};
+        launch_onesweep(&one, 1, bits, p * bits, 1 + p, ctx->stream, ctx->cfg.sort_block);
         cur ^= 1;
     }
     GS_CK(cudaGetLastError());

@@ -137,13 +137,15 @@ __global__ void k_frame_begin_multi(MultiViewFrames mv) {
 constexpr uint32_t kEmitItems = 8;                            // slots per thread of an emit chunk
 constexpr uint32_t kEmitChunk = kEmitItems * kScanThreads;    // slots per emit chunk
 template <uint32_t ITEMS>
-__global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __restrict__ counts,
-                                                            const uint4* __restrict__ meta, uint32_t n,
-                                                            uint32_t tiles_x, uint32_t max_instance,
-                                                            uint32_t digit_bits, uint32_t passes,
-                                                            uint32_t* __restrict__ offsets, uint32_t* __restrict__ keys,
-                                                            uint32_t* __restrict__ vals, FrameCtl* ctl,
-                                                            uint64_t* flags, uint32_t slot) {
+__device__ __forceinline__ void emit_view(const EmitView& view, uint32_t digit_bits, uint32_t slot) {
+    const uint32_t* __restrict__ const counts = view.counts;
+    const uint4* __restrict__ const meta = view.meta;
+    uint32_t* __restrict__ const offsets = view.offsets;
+    uint32_t* __restrict__ const keys = view.keys;
+    uint32_t* __restrict__ const vals = view.vals;
+    FrameCtl* const ctl = view.ctl;
+    uint64_t* const flags = view.flags;
+    const uint32_t n = view.n, tiles_x = view.tiles_x, max_instance = view.max_instance, passes = view.passes;
     constexpr uint32_t PART = ITEMS * kScanThreads;  // Gaussians per partition
     __shared__ uint32_t s_off[PART + 1];
     __shared__ uint2 s_meta[PART];  // (minX | minY << 16, rect width | depth16 << 16)
@@ -155,7 +157,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
     const uint32_t tid = threadIdx.x;
     const uint32_t radix = 1u << digit_bits;
     for (uint32_t i = tid; i < passes * radix; i += kScanThreads) s_hist[i] = 0u;
-    pdl_wait();  // also for the ticket counter, set two kernels back: see k_onesweep
     if (tid == 0) {
         s_part = atomicAdd(&ctl->tickets[slot], 1u);
         s_seq = ctl->seq + slot;
@@ -327,6 +328,21 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_emit(const uint32_t* __re
         if (s_hist[i]) atomicAdd(&ctl->hist[i], s_hist[i]);
 }
 
+// Both wait before they read anything, the ticket counter, set two kernels back, included: see k_onesweep.
+template <uint32_t ITEMS>
+__global__ void __launch_bounds__(kScanThreads) k_scan_emit(EmitView view, uint32_t digit_bits, uint32_t slot) {
+    pdl_wait();
+    emit_view<ITEMS>(view, digit_bits, slot);
+}
+template <uint32_t ITEMS>
+__global__ void __launch_bounds__(kScanThreads) k_scan_emit_views(const __grid_constant__ Views<EmitView> views,
+                                                                  uint32_t digit_bits, uint32_t slot) {
+    pdl_wait();
+    const EmitView& view = views.view[blockIdx.y];
+    if (blockIdx.x > view.n / (ITEMS * kScanThreads)) return;  // one CTA per partition of n + 1 entries
+    emit_view<ITEMS>(view, digit_bits, slot);
+}
+
 // ---- standalone exclusive scan (offset_scan.wgsl:22-67 semantics, any n) ------------------------
 __global__ void __launch_bounds__(kScanThreads) k_exclusive_scan(uint32_t* data, uint32_t n, uint32_t* total_out,
                                                                  FrameCtl* ctl, uint64_t* flags, uint32_t slot) {
@@ -447,17 +463,17 @@ __device__ __forceinline__ uint32_t sum_tagged(const uint64_t* p, size_t stride,
 //   - keys/values are staged in shared memory in local sorted order and written out at
 //     global_digit_base + rank, which keeps runs of equal digits contiguous in global memory.
 template <int BITS, int ITEMS, int SPLIT>
-__global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __restrict__ keys_in,
-                                                           const uint32_t* __restrict__ vals_in,
-                                                           uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-                                                           const uint32_t* n_dev, uint32_t n_host, uint32_t shift,
-                                                           uint32_t dmask, const uint32_t* __restrict__ hist,
-                                                           FrameCtl* ctl, uint64_t* flags, uint32_t slot,
-                                                           uint32_t* __restrict__ ranges, uint32_t tiles) {
-    // Nothing in global memory is read before the wait, not even what was written two kernels back (n, the
-    // histogram): a pass that took its ticket and digit bases early saw an unfinished histogram now and
-    // then when twenty views' sorts ran side by side in a graph (about 1 view in 300).
-    pdl_wait();
+__device__ __forceinline__ void sort_view(const SortView& view, uint32_t shift, uint32_t slot) {
+    const uint32_t* __restrict__ const keys_in = view.keys_in;
+    const uint32_t* __restrict__ const vals_in = view.vals_in;
+    uint32_t* __restrict__ const keys_out = view.keys_out;
+    uint32_t* __restrict__ const vals_out = view.vals_out;
+    const uint32_t* __restrict__ const hist = view.hist;
+    uint32_t* __restrict__ const ranges = view.ranges;
+    const uint32_t* const n_dev = view.n_dev;
+    FrameCtl* const ctl = view.ctl;
+    uint64_t* const flags = view.flags;
+    const uint32_t n_host = view.n_host, dmask = view.dmask, tiles = view.tiles;
     constexpr uint32_t RADIX = 1u << BITS;
     const uint32_t MASK = dmask & (RADIX - 1u);  // digit mask of this pass (narrower on a last partial digit)
     constexpr uint32_t WARPS = kSortThreads / 32;
@@ -621,6 +637,21 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const uint32_t* __
     }
 }
 
+// Nothing in global memory is read before the wait, not even what was written two kernels back (n, the
+// histogram): a pass that took its ticket and digit bases early saw an unfinished histogram now and
+// then when twenty views' sorts ran side by side in a graph (about 1 view in 300).
+template <int BITS, int ITEMS, int SPLIT>
+__global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(SortView view, uint32_t shift, uint32_t slot) {
+    pdl_wait();
+    sort_view<BITS, ITEMS, SPLIT>(view, shift, slot);
+}
+template <int BITS, int ITEMS, int SPLIT>
+__global__ void __launch_bounds__(kSortThreads, 4) k_onesweep_views(const __grid_constant__ Views<SortView> views,
+                                                                    uint32_t shift, uint32_t slot) {
+    pdl_wait();
+    sort_view<BITS, ITEMS, SPLIT>(views.view[blockIdx.y], shift, slot);
+}
+
 // ---- tile order: heaviest tiles first ----------------------------------------------------------------
 // The raster CTAs take their tiles from `order` (CTA i renders tile order[i]); CTAs start roughly in
 // index order, so listing the tiles by decreasing range length keeps the long tiles from forming the
@@ -660,9 +691,14 @@ __device__ __forceinline__ void slice_bins(const uint32_t* __restrict__ ranges, 
     }
 }
 
-__global__ void __launch_bounds__(kOrderThreads) k_tile_bins(const uint32_t* __restrict__ ranges, uint32_t tiles,
-                                                             uint32_t* __restrict__ slice_hist) {
+// (a single view is a batch of one here: the two kernels are all latency)
+__global__ void __launch_bounds__(kOrderThreads) k_tile_bins(const __grid_constant__ Views<OrderView> views) {
     pdl_wait();
+    const OrderView& view = views.view[blockIdx.y];
+    const uint32_t* const ranges = view.ranges;
+    const uint32_t tiles = view.tiles;
+    if (blockIdx.x * kOrderSlice >= tiles) return;
+    uint32_t* const slice_hist = view.slice_hist;
     __shared__ uint32_t s_bin[65];
     if (threadIdx.x < 65u) s_bin[threadIdx.x] = 0u;
     __syncthreads();
@@ -674,13 +710,17 @@ __global__ void __launch_bounds__(kOrderThreads) k_tile_bins(const uint32_t* __r
     if (threadIdx.x < 64u) slice_hist[blockIdx.x * 64u + threadIdx.x] = s_bin[threadIdx.x];
 }
 
-__global__ void __launch_bounds__(kOrderThreads) k_tile_place(uint32_t* __restrict__ ranges, uint32_t tiles,
-                                                              const uint32_t* __restrict__ slice_hist,
-                                                              uint32_t* __restrict__ order, uint32_t* status) {
+__global__ void __launch_bounds__(kOrderThreads) k_tile_place(const __grid_constant__ Views<OrderView> views) {
     pdl_wait();
+    const OrderView& view = views.view[blockIdx.y];
+    uint32_t* const ranges = view.ranges;
+    const uint32_t tiles = view.tiles;
+    if (blockIdx.x * kOrderSlice >= tiles) return;
+    const uint32_t* const slice_hist = view.slice_hist;
+    uint32_t *const order = view.order, *const status = view.status;
     __shared__ uint32_t s_incl[64];
     __shared__ uint32_t s_base[64];
-    const uint32_t tid = threadIdx.x, slices = gridDim.x;
+    const uint32_t tid = threadIdx.x, slices = (tiles + kOrderSlice - 1u) / kOrderSlice;
     uint32_t b[kOrderPer];
     slice_bins(ranges, tiles, blockIdx.x, b);  // in flight while the table is summed
     uint32_t total = 0, before = 0, incl = 0;
@@ -755,13 +795,13 @@ void launch_frame_begin(FrameCtl* ctl, uint64_t* flags, uint32_t flag_words, cud
     launch_pdl(k_frame_begin, dim3(grid), dim3(256), s, ctl, ranges, range_words, flags, flag_words);
 }
 
-void launch_scan_emit(const uint32_t* counts, const uint4* meta, uint32_t n, uint32_t tiles_x, uint32_t max_instance,
-                      uint32_t digit_bits, uint32_t passes, uint32_t* offsets, uint32_t* keys, uint32_t* vals,
-                      FrameCtl* ctl, uint64_t* flags, uint32_t slot, cudaStream_t s) {
-    auto launch = [&](auto kernel, uint32_t items) {
+void launch_scan_emit(const EmitView* views, uint32_t count, uint32_t digit_bits, uint32_t slot, cudaStream_t s) {
+    uint32_t n = 0;
+    for (uint32_t v = 0; v < count; ++v) n = std::max(n, views[v].n);
+    auto launch = [&](auto kernel, auto kernel_views, uint32_t items) {
         const uint32_t part = items * kScanThreads, parts = (uint32_t)(((uint64_t)n + part) / part);  // n + 1 entries
-        launch_pdl(kernel, dim3(parts), dim3(kScanThreads), s, counts, meta, n, tiles_x, max_instance, digit_bits, passes,
-                   offsets, keys, vals, ctl, flags, slot);
+        if (count == 1) launch_pdl(kernel, dim3(parts), dim3(kScanThreads), s, views[0], digit_bits, slot);
+        else launch_pdl(kernel_views, dim3(parts, count), dim3(kScanThreads), s, pack_views(views, count), digit_bits, slot);
     };
     // The emit of a partition is one CTA's work, so a small scene needs small partitions to fill the GPU (a
     // close-up's Gaussians emit dozens of instances each), while the predecessor sums and the histograms' global
@@ -769,10 +809,11 @@ void launch_scan_emit(const uint32_t* counts, const uint4* meta, uint32_t n, uin
     // 512x512 13.8 / 13.2 / 15.7 / 28.5, a close-up of 60k 27.8 / 37.6 / 54 / 99, 100k at 320x240 14.5 / 13.6 /
     // 12.3 / 19.0, 250k in 8x8 tiles 31 / 26 / 24.7 / 32.4, 500k 44 / 30 / 17.8 / 19.8, 1M 80 / 49 / 28.9 / 30.8,
     // 3M at 4K - / - / 97 / 113, 8M - / - / 171 / 164, 16M - / - / 365 / 344
-    if (n < 75000u) launch(k_scan_emit<1>, 1u);
-    else if (n < 150000u) launch(k_scan_emit<2>, 2u);
-    else if (n < 8000000u) launch(k_scan_emit<4>, 4u);
-    else launch(k_scan_emit<8>, 8u);
+    const uint64_t all = (uint64_t)n * count;  // several views fill the GPU together
+    if (all < 75000u) launch(k_scan_emit<1>, k_scan_emit_views<1>, 1u);
+    else if (all < 150000u) launch(k_scan_emit<2>, k_scan_emit_views<2>, 2u);
+    else if (n < 8000000u) launch(k_scan_emit<4>, k_scan_emit_views<4>, 4u);
+    else launch(k_scan_emit<8>, k_scan_emit_views<8>, 8u);
 }
 
 void launch_exclusive_scan(uint32_t* data, uint32_t n, uint32_t* total_dev, FrameCtl* ctl, uint64_t* flags,
@@ -792,32 +833,31 @@ void launch_digit_hist(const uint32_t* keys, uint32_t n, uint32_t digit_bits, ui
 
 void configure_sort_kernels() {
     // the largest shared-memory carveout lets more onesweep CTAs (up to 44 KB each) share an SM
-    cudaFuncSetAttribute(k_onesweep<4, 8, 0>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<4, 16, 0>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<8, 8, 0>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<8, 8, 2>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<8, 8, 3>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<8, 8, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<8, 16, 0>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<8, 16, 2>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<8, 16, 3>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaFuncSetAttribute(k_onesweep<8, 16, 4>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+#define GS_CARVEOUT(B, I, S)                                                                            \
+    cudaFuncSetAttribute(k_onesweep<B, I, S>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);     \
+    cudaFuncSetAttribute(k_onesweep_views<B, I, S>, cudaFuncAttributePreferredSharedMemoryCarveout, 100)
+    GS_CARVEOUT(4, 8, 0); GS_CARVEOUT(4, 16, 0);
+    GS_CARVEOUT(8, 8, 0); GS_CARVEOUT(8, 8, 2); GS_CARVEOUT(8, 8, 3); GS_CARVEOUT(8, 8, 4);
+    GS_CARVEOUT(8, 16, 0); GS_CARVEOUT(8, 16, 2); GS_CARVEOUT(8, 16, 3); GS_CARVEOUT(8, 16, 4);
+#undef GS_CARVEOUT
 }
 
-void launch_onesweep(uint32_t digit_bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
-                     uint32_t* vals_out, const uint32_t* n_dev, uint32_t n_host, uint32_t max_n, uint32_t shift,
-                     uint32_t dmask, const uint32_t* hist, FrameCtl* ctl, uint64_t* flags, uint32_t slot,
-                     int grid_cap, cudaStream_t s, uint32_t block, uint32_t split, uint32_t* ranges,
-                     uint32_t tiles) {
+void launch_onesweep(const SortView* views, uint32_t count, uint32_t digit_bits, uint32_t shift, uint32_t slot,
+                     cudaStream_t s, uint32_t block, uint32_t split) {
     const bool small = block == kSortPartitionMin;
     const uint32_t part = small ? kSortPartitionMin : kSortPartition;
-    uint32_t parts = (max_n + part - 1u) / part;
-    const uint32_t cap = grid_cap > 0 ? (uint32_t)grid_cap : (uint32_t)sm_count() * 4u;
-    if (parts > cap) parts = cap;
+    uint32_t parts = 0;
+    for (uint32_t v = 0; v < count; ++v) parts = std::max(parts, (uint32_t)(((uint64_t)views[v].max_n + part - 1u) / part));
+    // the CTAs that fit at once; several views share them (a CTA goes on with the view's next partition)
+    const uint32_t fit = (uint32_t)sm_count() * 4u;
+    parts = std::min(parts, count == 1 ? fit : std::max(2u * fit / count, fit / 4u));
     if (parts == 0) parts = 1;
-#define GS_ONESWEEP(B, I, S)                                                                                      \
-    launch_pdl(k_onesweep<B, I, S>, dim3(parts), dim3(kSortThreads), s, keys_in, vals_in, keys_out, vals_out, n_dev, \
-               n_host, shift, dmask, hist, ctl, flags, slot, ranges, tiles)
+#define GS_ONESWEEP(B, I, S)                                                                                     \
+    do {                                                                                                         \
+        if (count == 1) launch_pdl(k_onesweep<B, I, S>, dim3(parts), dim3(kSortThreads), s, views[0], shift, slot); \
+        else launch_pdl(k_onesweep_views<B, I, S>, dim3(parts, count), dim3(kSortThreads), s,                     \
+                        pack_views(views, count), shift, slot);                                                  \
+    } while (0)
 #define GS_ONESWEEP_SPLIT(I)                             \
     switch (split) {                                     \
         case 2: GS_ONESWEEP(8, I, 2); break;             \
@@ -840,13 +880,12 @@ void launch_check_canaries(const CanaryList& list, uint32_t* status, cudaStream_
 
 uint32_t tile_order_slices(uint32_t tiles) { return (tiles + kOrderSlice - 1u) / kOrderSlice; }
 
-void launch_tile_order(uint32_t* ranges, uint32_t tiles, uint32_t* slice_hist, uint32_t* order, uint32_t* status,
-                       cudaStream_t s) {
-    const uint32_t slices = std::max(1u, tile_order_slices(tiles));
-    launch_pdl(k_tile_bins, dim3(slices), dim3(kOrderThreads), s, ranges, tiles, slice_hist);
-    launch_pdl(k_tile_place, dim3(slices), dim3(kOrderThreads), s, ranges, tiles, (const uint32_t*)slice_hist, order,
-               status);
+void launch_tile_order(const OrderView* views, uint32_t count, cudaStream_t s) {
+    uint32_t slices = 1;
+    for (uint32_t v = 0; v < count; ++v) slices = std::max(slices, tile_order_slices(views[v].tiles));
+    const Views<OrderView> p = pack_views(views, count);
+    launch_pdl(k_tile_bins, dim3(slices, count), dim3(kOrderThreads), s, p);
+    launch_pdl(k_tile_place, dim3(slices, count), dim3(kOrderThreads), s, p);
 }
-
 
 }  // namespace gs

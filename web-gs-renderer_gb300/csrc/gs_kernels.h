@@ -54,6 +54,20 @@ void launch_frame_begin(FrameCtl* ctl, uint64_t* flags, uint32_t flag_words, cud
 // Up to kMaxMultiViews views of one scene for launch_preprocess_multi: each view's block and frame
 // outputs.
 constexpr uint32_t kMaxMultiViews = 16;
+// Views that one launch of the later stages takes, as its kernel parameter (the rule: views_per_run).
+constexpr uint32_t kMaxRunViews = 8;
+template <class V>
+struct Views {
+    V view[kMaxRunViews];
+    uint32_t count;
+};
+template <class V>
+inline Views<V> pack_views(const V* views, uint32_t count) {
+    Views<V> p{};
+    for (uint32_t i = 0; i < count; ++i) p.view[i] = views[i];
+    p.count = count;
+    return p;
+}
 struct MultiViewFrames {
     const ViewBlock* view[kMaxMultiViews];
     float4* rec[kMaxMultiViews];
@@ -81,9 +95,18 @@ constexpr uint32_t kScanItems = 8;
 constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanPartition = kScanItems * kScanThreads;
 constexpr uint32_t kEmitPartitionMin = kScanThreads;  // smallest partition of launch_scan_emit
-void launch_scan_emit(const uint32_t* counts, const uint4* meta, uint32_t n, uint32_t tiles_x, uint32_t max_instance,
-                      uint32_t digit_bits, uint32_t passes, uint32_t* offsets, uint32_t* keys, uint32_t* vals,
-                      FrameCtl* ctl, uint64_t* flags, uint32_t slot, cudaStream_t s);
+
+// The binning and raster launches take one view, or up to kMaxRunViews views of a batch at once: one
+// launch per stage for all of them, a row of CTAs per view. count 1 is the plain frame.
+struct EmitView {
+    const uint32_t* counts;
+    const uint4* meta;
+    uint32_t *offsets, *keys, *vals;
+    FrameCtl* ctl;
+    uint64_t* flags;
+    uint32_t n, tiles_x, max_instance, passes;
+};
+void launch_scan_emit(const EmitView* views, uint32_t count, uint32_t digit_bits, uint32_t slot, cudaStream_t s);
 
 // Onesweep LSD radix pass. n comes from *n_dev when non-null, else n_host. flags must hold
 // onesweep_flag_words(partitions, radix) words for the largest partition count the pass can see (the
@@ -102,11 +125,18 @@ constexpr uint32_t kSortPartition = kSortThreads * kSortItems; // largest sort b
 constexpr uint32_t kSortPartitionMin = kSortThreads * 8;       // smallest sort block (2048 keys)
 // Per-device kernel attributes (shared-memory carveout of the sort); call once per context.
 void configure_sort_kernels();
-void launch_onesweep(uint32_t digit_bits, const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
-                     uint32_t* vals_out, const uint32_t* n_dev, uint32_t n_host, uint32_t max_n, uint32_t shift,
-                     uint32_t dmask, const uint32_t* hist, FrameCtl* ctl, uint64_t* flags, uint32_t slot,
-                     int grid_cap, cudaStream_t s, uint32_t block = kSortPartition, uint32_t split = 0,
-                     uint32_t* ranges = nullptr, uint32_t tiles = 0);
+struct SortView {
+    const uint32_t *keys_in, *vals_in;
+    uint32_t *keys_out, *vals_out;
+    const uint32_t* n_dev;
+    const uint32_t* hist;
+    FrameCtl* ctl;
+    uint64_t* flags;
+    uint32_t* ranges;
+    uint32_t n_host, max_n, dmask, tiles;
+};
+void launch_onesweep(const SortView* views, uint32_t count, uint32_t digit_bits, uint32_t shift, uint32_t slot,
+                     cudaStream_t s, uint32_t block = kSortPartition, uint32_t split = 0);
 // ranges (the last pass of a frame's sort only): each tile's (first, last + 1) in the sorted keys is
 // combined into ranges[2 tile], ranges[2 tile + 1] by atomic min / max over the CTAs; the ranges must
 // hold (0xFFFFFFFF, 0) before the pass (launch_frame_begin) and launch_tile_order, which reads them
@@ -123,8 +153,12 @@ void launch_exclusive_scan(uint32_t* data, uint32_t n, uint32_t* total_dev, Fram
 // kernels over slices of 1024 tiles. slice_hist holds 64 words per slice (tile_order_slices), fully
 // rewritten by every call.
 uint32_t tile_order_slices(uint32_t tiles);
-void launch_tile_order(uint32_t* ranges, uint32_t tiles, uint32_t* slice_hist, uint32_t* order, uint32_t* status,
-                       cudaStream_t s);
+struct OrderView {
+    uint32_t* ranges;
+    uint32_t *slice_hist, *order, *status;
+    uint32_t tiles;
+};
+void launch_tile_order(const OrderView* views, uint32_t count, cudaStream_t s);
 
 // Checked builds: verifies the canary pads of up to kCanaryListMax buffers (head and tail pad of
 // kCanaryBytes each, filled with kCanaryWord) and sets kDevCanary in *status if any word changed.
@@ -157,9 +191,15 @@ __host__ __device__ __forceinline__ size_t hit_mask_base(uint32_t start, uint32_
 // positions culled per step (32 to 256). ctl (optional) bounds every range by the sorted count; n bounds the Gaussian indices; order
 // (optional) is the tile each CTA renders (launch_tile_order), else CTA i renders tile i.
 void configure_raster_kernels();
-void launch_raster(uint32_t tile, uint32_t batch, const uint32_t* ranges, const uint32_t* vals, const float4* rec,
-                   uint32_t n, const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x,
-                   uint32_t tiles_y, const RasterOut& out, const uint32_t* order, cudaStream_t s);
+struct RasterView {
+    const uint32_t *ranges, *vals;
+    const float4* rec;
+    const FrameCtl* ctl;
+    const uint32_t* order;
+    RasterOut out;
+    uint32_t n, width, height, tiles_x, tiles;
+};
+void launch_raster(const RasterView* views, uint32_t count, uint32_t tile, uint32_t batch, cudaStream_t s);
 
 // y = the pinned exp of x (raster: the raster's exp, defined on [-5.6, 0]).
 void launch_exp(const float* x, float* y, uint32_t n, cudaStream_t s, bool raster = false);

@@ -38,6 +38,8 @@
 // Tiles start in order[]'s order: by decreasing range length, so the longest tiles
 // start first instead of forming the tail of the launch (with tiles in index order the clustered
 // scenes left about a third of the launch time to a few long tiles).
+#include <algorithm>
+
 #include "gs_kernels.h"
 #include "gs_raster_common.cuh"
 
@@ -124,19 +126,22 @@ __device__ __forceinline__ void blend_one(float power, float alpha, float one_mi
 }
 #undef GS_BLEND
 
+// The CTA of sub-block `sub` of the tile at place `at` of the view's order.
 template <int TILE, int KEEP>
-__global__ void __launch_bounds__(RasterShared<TILE>::kWarps * 32, 32 / RasterShared<TILE>::kWarps)
-k_raster(const uint32_t* __restrict__ ranges, const uint32_t* __restrict__ vals, const float4* __restrict__ rec,
-         uint32_t n, const FrameCtl* __restrict__ ctl, uint32_t width, uint32_t height, uint32_t tiles_x, RasterOut out,
-         const uint32_t* __restrict__ order, uint32_t step) {
-    pdl_wait();
+__device__ __forceinline__ void raster_view(const RasterView& view, uint32_t at, uint32_t sub, uint32_t step) {
+    const uint32_t* __restrict__ const ranges = view.ranges;
+    const uint32_t* __restrict__ const vals = view.vals;
+    const float4* __restrict__ const rec = view.rec;
+    const FrameCtl* __restrict__ const ctl = view.ctl;
+    const uint32_t* __restrict__ const order = view.order;
+    const RasterOut out = view.out;
+    const uint32_t n = view.n, width = view.width, height = view.height, tiles_x = view.tiles_x;
     constexpr bool LAST = KEEP == kKeepLast;
     constexpr uint32_t kSub = RasterShared<TILE>::kSub, kWarps = RasterShared<TILE>::kWarps, kThreads = 32u * kWarps;
     constexpr uint32_t kSubs = TILE / kSub;  // CTAs across the tile
     extern __shared__ __align__(16) unsigned char s_raw[];
     RasterShared<TILE>& cta = *reinterpret_cast<RasterShared<TILE>*>(s_raw);
 
-    const uint32_t sub = blockIdx.x % (kSubs * kSubs), at = blockIdx.x / (kSubs * kSubs);
     const uint32_t tile = order ? order[at] : at;
     const uint32_t px0 = (tile % tiles_x) * TILE + kSub * (sub % kSubs), py0 = (tile / tiles_x) * TILE + kSub * (sub / kSubs);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -267,7 +272,7 @@ k_raster(const uint32_t* __restrict__ ranges, const uint32_t* __restrict__ vals,
         out.rgb[3 * p + 2] = cb;
     }
     if (KEEP != kKeepNothing && out.final_t) out.final_t[p] = final_t;
-    if (LAST) out.n_contrib[p] = last;
+    if (LAST && out.n_contrib) out.n_contrib[p] = last;
     if (out.rgba8) {
         const uint32_t r8 = (uint32_t)(fminf(fmaxf(cr, 0.0f), 1.0f) * 255.0f + 0.5f);
         const uint32_t g8 = (uint32_t)(fminf(fmaxf(cg, 0.0f), 1.0f) * 255.0f + 0.5f);
@@ -276,19 +281,44 @@ k_raster(const uint32_t* __restrict__ ranges, const uint32_t* __restrict__ vals,
     }
 }
 
+template <int TILE, int KEEP>
+__global__ void __launch_bounds__(RasterShared<TILE>::kWarps * 32, 32 / RasterShared<TILE>::kWarps)
+k_raster(RasterView view, uint32_t step) {
+    pdl_wait();
+    constexpr uint32_t kSubs = (TILE / RasterShared<TILE>::kSub) * (TILE / RasterShared<TILE>::kSub);
+    raster_view<TILE, KEEP>(view, blockIdx.x / kSubs, blockIdx.x % kSubs, step);
+}
+// Several views: their longest tiles first, view by view, then their next ones.
+template <int TILE, int KEEP>
+__global__ void __launch_bounds__(RasterShared<TILE>::kWarps * 32, 32 / RasterShared<TILE>::kWarps)
+k_raster_views(const __grid_constant__ Views<RasterView> views, uint32_t step) {
+    pdl_wait();
+    constexpr uint32_t kSubs = (TILE / RasterShared<TILE>::kSub) * (TILE / RasterShared<TILE>::kSub);
+    const uint32_t unit = blockIdx.x / kSubs, at = unit / views.count;
+    const RasterView& view = views.view[unit % views.count];
+    if (at >= view.tiles) return;
+    raster_view<TILE, KEEP>(view, at, blockIdx.x % kSubs, step);
+}
+
 template <int TILE>
-void launch_tile(uint32_t step, const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n,
-                 const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
-                 const RasterOut& out, const uint32_t* order, cudaStream_t s) {
+void launch_tile(const RasterView* views, uint32_t count, uint32_t step, cudaStream_t s) {
     constexpr uint32_t kSubs = TILE / RasterShared<TILE>::kSub;
-    const dim3 grid(tiles_x * tiles_y * kSubs * kSubs), block(RasterShared<TILE>::kWarps * 32);
+    uint32_t tiles = 0;
+    bool last = false, final_t = false;
+    for (uint32_t v = 0; v < count; ++v) {
+        tiles = std::max(tiles, views[v].tiles);
+        last = last || views[v].out.n_contrib;
+        final_t = final_t || views[v].out.final_t;
+    }
+    const dim3 grid(tiles * count * kSubs * kSubs), block(RasterShared<TILE>::kWarps * 32);
     const size_t smem = sizeof(RasterShared<TILE>);
-    auto launch = [&](auto kernel) {
-        launch_pdl_smem(kernel, grid, block, smem, s, ranges, vals, rec, n, ctl, width, height, tiles_x, out, order, step);
+    auto launch = [&](auto kernel, auto kernel_views) {
+        if (count == 1) launch_pdl_smem(kernel, grid, block, smem, s, views[0], step);
+        else launch_pdl_smem(kernel_views, grid, block, smem, s, pack_views(views, count), step);
     };
-    if (out.n_contrib) launch(k_raster<TILE, kKeepLast>);
-    else if (out.final_t) launch(k_raster<TILE, kKeepT>);
-    else launch(k_raster<TILE, kKeepNothing>);
+    if (last) launch(k_raster<TILE, kKeepLast>, k_raster_views<TILE, kKeepLast>);
+    else if (final_t) launch(k_raster<TILE, kKeepT>, k_raster_views<TILE, kKeepT>);
+    else launch(k_raster<TILE, kKeepNothing>, k_raster_views<TILE, kKeepNothing>);
 }
 
 template <int TILE>
@@ -300,6 +330,9 @@ void configure_tile() {
     configure(k_raster<TILE, kKeepNothing>);
     configure(k_raster<TILE, kKeepT>);
     configure(k_raster<TILE, kKeepLast>);
+    configure(k_raster_views<TILE, kKeepNothing>);
+    configure(k_raster_views<TILE, kKeepT>);
+    configure(k_raster_views<TILE, kKeepLast>);
 }
 
 }  // namespace
@@ -310,13 +343,11 @@ void configure_raster_kernels() {
     configure_tile<32>();
 }
 
-void launch_raster(uint32_t tile, uint32_t batch, const uint32_t* ranges, const uint32_t* vals, const float4* rec,
-                   uint32_t n, const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x,
-                   uint32_t tiles_y, const RasterOut& out, const uint32_t* order, cudaStream_t s) {
+void launch_raster(const RasterView* views, uint32_t count, uint32_t tile, uint32_t batch, cudaStream_t s) {
     batch *= 4u;  // positions per cull step (128 to 1024, a multiple of 32): most tiles need one step
-    if (tile == 8) launch_tile<8>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s);
-    else if (tile == 32) launch_tile<32>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s);
-    else launch_tile<16>(batch, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_y, out, order, s);
+    if (tile == 8) launch_tile<8>(views, count, batch, s);
+    else if (tile == 32) launch_tile<32>(views, count, batch, s);
+    else launch_tile<16>(views, count, batch, s);
 }
 
 }  // namespace gs
