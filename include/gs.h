@@ -74,8 +74,8 @@ typedef struct gs_camera {
 typedef struct gs_config {
     uint32_t tile_size;           /* 16 (reference); 8 and 32 also supported */
     uint32_t digit_bits;          /* radix digit width: 8 (reference) or 4 */
-    uint32_t raster_batch;        /* raster depth: 32, 64, 128 or 256; a CTA culls four times as many splats
-                                     at a time */
+    uint32_t raster_batch;        /* raster depth: 32, 64, 128 or 256; a CTA stages up to four times as many
+                                     splats at a time */
     uint32_t max_instance_factor; /* instance budget per Gaussian (MAX_INSTANCE_FACTOR = 64) */
     uint32_t flags;               /* GS_FLAG_* */
     int32_t device;               /* CUDA device ordinal */

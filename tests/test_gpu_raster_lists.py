@@ -1,6 +1,6 @@
 """The raster against the oracle, bit for bit, at list lengths on both sides of what it handles at once
-(pairs, 16 and 32 hits per step, a ring of 64, groups of 32 positions, cull steps of 128 and 1024), in every
-tile size: faint splats, so that every list is walked to its end, and opaque ones, so that pixels end at
+(pairs, 32 hits per chunk, a list of 64, groups of 32 positions, steps of 128 and 512), in every tile
+size: faint splats, so that every list is walked to its end, and opaque ones, so that pixels end at
 different places of it."""
 import numpy as np
 import pytest
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("tile", [8, 16, 32])
 @pytest.mark.parametrize("logit", [-3.0, 2.0])
-@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 31, 33, 64, 65, 127, 129, 700, 1100])
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 31, 32, 33, 64, 65, 127, 129, 512, 513, 700, 1100])
 def test_list_lengths(n, logit, tile):
     packed = W.SceneSpec(n, 900 + n, 0).build()
     packed[:3 * n] *= 0.3

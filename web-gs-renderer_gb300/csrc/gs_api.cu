@@ -93,7 +93,7 @@ struct Frame {
     DevBuf<uint32_t> keys[2], vals[2];
     DevBuf<uint64_t> flags;
     DevBuf<uint32_t> ranges;
-    DevBuf<uint32_t> order;  // tiles by decreasing range length: the raster CTAs' tile order
+    DevBuf<uint4> order;  // tiles and ranges by decreasing length: the raster CTAs' tile order
     DevBuf<uint32_t> order_hist;  // per-slice bin counts of the tile order (64 words per 1024 tiles)
     DevBuf<uint32_t> rgba8, n_contrib;
     DevBuf<uint32_t> hit_masks;  // differentiable frames: the raster's hits per 8x4 block (RasterOut)
@@ -353,9 +353,11 @@ RasterOut raster_out(const gs_ctx* ctx, Frame& f, const gs_image* out, size_t ma
     return ro;
 }
 
-// Enqueues the passes after the preprocess (renderer.js:836-932) of `count` frames (1 to kMaxRunViews) on stream s,
-// every stage one launch for all of them. profile: events around the stages, from kPassScanEmit on.
-void enqueue_views(gs_ctx* ctx, Frame* const* frames, const FrameArgs* args, uint32_t count, cudaStream_t s, bool profile) {
+// Enqueues the passes after the preprocess (renderer.js:836-932) of `count` frames (1 to kMaxRunViews) on
+// stream s, every stage one launch for all of them; together: with the views that run beside them on other
+// streams. profile: events around the stages, from kPassScanEmit on.
+void enqueue_views(gs_ctx* ctx, Frame* const* frames, const FrameArgs* args, uint32_t count, uint32_t together,
+                   cudaStream_t s, bool profile) {
     const uint32_t bits = ctx->cfg.digit_bits, radix = 1u << bits;
     EmitView emit[kMaxRunViews];
     OrderView order[kMaxRunViews];
@@ -367,12 +369,12 @@ void enqueue_views(gs_ctx* ctx, Frame* const* frames, const FrameArgs* args, uin
         const uint32_t tiles = a.tiles_x * a.tiles_y, sorted = a.passes & 1u;
         emit[v] = EmitView{f.counts.p, f.meta.p, f.offsets.p, f.keys[0].p, f.vals[0].p, f.ctl.p, f.flags.p,
                            a.n, a.tiles_x, a.max_instance, a.passes};
-        order[v] = OrderView{f.ranges.p, f.order_hist.p, f.order.p, &f.ctl.p->status, tiles};
-        raster[v] = RasterView{f.ranges.p, f.vals[sorted].p, f.rec.p, f.ctl.p, f.order.p, a.out, a.n, a.w, a.h, a.tiles_x, tiles};
+        order[v] = OrderView{f.ranges.p, f.order_hist.p, f.order.p, f.ctl.p, tiles};
+        raster[v] = RasterView{f.order.p, f.vals[sorted].p, f.rec.p, a.out, a.n, a.w, a.h, a.tiles_x, tiles};
         passes = std::max(passes, a.passes);
         key_bits = std::max(key_bits, 16u + bitlen(tiles - 1u));
     }
-    launch_scan_emit(emit, count, bits, 0, s);
+    launch_scan_emit(emit, count, together, bits, 0, s);
     if (profile) cudaEventRecord(ctx->ev[kPassScanEmit + 1], s);
     for (uint32_t p = 0; p < passes; ++p) {
         // the tile digits arrive in depth order, nearly all distinct within a warp: their ranking
@@ -410,7 +412,7 @@ void enqueue_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a, cudaStream_t s, bo
                       f.ctl.p, s);
     if (profile) cudaEventRecord(ctx->ev[kPassPreprocess + 1], s);
     Frame* const one = &f;
-    enqueue_views(ctx, &one, &a, 1, s, profile);
+    enqueue_views(ctx, &one, &a, 1, 1, s, profile);
 }
 
 void remember(Frame& f, const FrameArgs& a) {
@@ -522,7 +524,7 @@ int capture_and_launch(gs_ctx* ctx, cudaGraphExec_t* exec, GraphKey* cached, con
                         s = ctx->side[next++ % used];
                         cudaStreamWaitEvent(s, ctx->views_ready, 0);
                     }
-                    enqueue_views(ctx, group + v, group_args + v, std::min(run, mv.count - v), s, false);
+                    enqueue_views(ctx, group + v, group_args + v, std::min(run, mv.count - v), mv.count, s, false);
                 }
             }
             for (int s = 0; s < used; ++s) {
@@ -1061,9 +1063,9 @@ static int enqueue_raster_backward(gs_ctx* ctx, Frame& f, const gs_scene* scene,
     if (scene->n && !f.grad2d_zero) GS_CK(cudaMemsetAsync(f.grad2d.p, 0, f.grad2d.cap * sizeof(float), s));
     f.grad2d_zero = false;
     if (ev) cudaEventRecord(ev[0], s);
-    launch_raster_backward(ctx->cfg.tile_size, f.ranges.p, f.vals[f.sorted_buf].p, f.rec.p, scene->n, f.ctl.p, f.width,
+    launch_raster_backward(ctx->cfg.tile_size, f.order.p, f.vals[f.sorted_buf].p, f.rec.p, scene->n, f.width,
                            f.height, f.tiles_x, f.tiles_y, f.final_t.p, f.n_contrib.p, f.hit_masks.p, f.mask_pitch, dl,
-                           f.grad2d.p, f.order.p, s);
+                           f.grad2d.p, s);
     if (ev) cudaEventRecord(ev[1], s);
     GS_CK(cudaGetLastError());
     return GS_OK;

@@ -211,10 +211,9 @@ struct BwdWarp {
 // branch in a hit 664; columns without selects and predicated atomics 631; heads by integer rounding 603;
 // hits in pairs on packed operations 577, their loop fully unrolled 560.
 template <int TILE>
-__global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backward(const uint32_t* __restrict__ ranges,
+__global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backward(const uint4* __restrict__ order,
                                                                      const uint32_t* __restrict__ vals,
                                                                      const float4* __restrict__ rec, uint32_t n,
-                                                                     const FrameCtl* __restrict__ ctl,
                                                                      uint32_t width, uint32_t height,
                                                                      uint32_t tiles_x, uint32_t tiles,
                                                                      const float* __restrict__ final_t,
@@ -222,8 +221,7 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
                                                                      const uint32_t* __restrict__ hit_masks,
                                                                      size_t mask_pitch,
                                                                      const float* __restrict__ dl_drgb,
-                                                                     float* __restrict__ grad2d,
-                                                                     const uint32_t* __restrict__ order) {
+                                                                     float* __restrict__ grad2d) {
     pdl_wait();
     constexpr uint32_t WX = TILE / 8, kTileWarps = TILE * TILE / 32;
     constexpr float kCx = 3.5f, kCy = 1.5f;  // centre of a warp's block
@@ -234,12 +232,10 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
     const uint32_t wid = blockIdx.x * kBwdWarps + (threadIdx.x >> 5);
     const uint32_t warp = wid % kTileWarps;
     if (wid / kTileWarps >= tiles) return;
-    const uint32_t tile = order ? order[wid / kTileWarps] : wid / kTileWarps;
+    const uint4 place = __ldg(order + wid / kTileWarps);
+    const uint32_t tile = place.x, start = place.y, end = place.z;
     const uint32_t tx = tile % tiles_x, ty = tile / tiles_x;
     const uint32_t bx0 = tx * TILE + 8u * (warp % WX), by0 = ty * TILE + 4u * (warp / WX);
-    const uint2 range = reinterpret_cast<const uint2*>(ranges)[tile];
-    const uint32_t end = ctl ? min(range.y, ctl->sorted_count) : range.y;
-    const uint32_t start = range.x;
     const uint32_t len = end > start ? end - start : 0u;
 
     PixState p;
@@ -416,14 +412,13 @@ void configure_raster_backward() {
     cudaFuncSetAttribute(k_raster_backward<32>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
 }
 
-void launch_raster_backward(uint32_t tile, const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n,
-                            const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
+void launch_raster_backward(uint32_t tile, const uint4* order, const uint32_t* vals, const float4* rec, uint32_t n,
+                            uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
                             const float* final_t, const uint32_t* n_contrib, const uint32_t* hit_masks,
-                            size_t mask_pitch, const float* dl_drgb, float* grad2d, const uint32_t* order,
-                            cudaStream_t s) {
+                            size_t mask_pitch, const float* dl_drgb, float* grad2d, cudaStream_t s) {
     auto launch = [&](auto bwd) {
-        bwd(tiles_x * tiles_y, s, ranges, vals, rec, n, ctl, width, height, tiles_x, tiles_x * tiles_y, final_t, n_contrib,
-            hit_masks, mask_pitch, dl_drgb, grad2d, order);
+        bwd(tiles_x * tiles_y, s, order, vals, rec, n, width, height, tiles_x, tiles_x * tiles_y, final_t, n_contrib,
+            hit_masks, mask_pitch, dl_drgb, grad2d);
     };
     if (tile == 8) launch([](auto&&... a) { launch_bwd_tile<8>(a...); });
     else if (tile == 32) launch([](auto&&... a) { launch_bwd_tile<32>(a...); });

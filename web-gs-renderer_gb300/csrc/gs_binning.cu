@@ -653,7 +653,9 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep_views(const __grid
 }
 
 // ---- tile order: heaviest tiles first ----------------------------------------------------------------
-// The raster CTAs take their tiles from `order` (CTA i renders tile order[i]); CTAs start roughly in
+// The raster CTAs take their tiles from `order`, (tile, first, last + 1, 0) in the sorted instances: the tile
+// with its range, so that a CTA's first load is not followed by one for the range (a tile of a dozen
+// instances is little else than the chain of its loads). CTA i renders order[i]; CTAs start roughly in
 // index order, so listing the tiles by decreasing range length keeps the long tiles from forming the
 // tail of the launch. Lengths are binned (four bins per octave, 64 bins, longest first) and placed by
 // a counting sort; the order inside a bin is whatever the atomics give and changes no output, since
@@ -674,11 +676,10 @@ constexpr uint32_t kOrderThreads = 256;
 constexpr uint32_t kOrderPer = 4;                                  // tiles per thread
 constexpr uint32_t kOrderSlice = kOrderThreads * kOrderPer;        // tiles per CTA
 
-// the bins of the calling thread's kOrderPer tiles of slice `slice` (64 for tiles past the end);
-// all loads are issued before any is used
+// the ranges of the calling thread's kOrderPer tiles of slice `slice` and their bins (64 for tiles past the
+// end); all loads are issued before any is used
 __device__ __forceinline__ void slice_bins(const uint32_t* __restrict__ ranges, uint32_t tiles, uint32_t slice,
-                                           uint32_t b[kOrderPer]) {
-    uint2 r[kOrderPer];
+                                           uint2 r[kOrderPer], uint32_t b[kOrderPer]) {
 #pragma unroll
     for (uint32_t k = 0; k < kOrderPer; ++k) {
         const uint32_t t = slice * kOrderSlice + k * kOrderThreads + threadIdx.x;
@@ -702,8 +703,9 @@ __global__ void __launch_bounds__(kOrderThreads) k_tile_bins(const __grid_consta
     __shared__ uint32_t s_bin[65];
     if (threadIdx.x < 65u) s_bin[threadIdx.x] = 0u;
     __syncthreads();
+    uint2 r[kOrderPer];
     uint32_t b[kOrderPer];
-    slice_bins(ranges, tiles, blockIdx.x, b);
+    slice_bins(ranges, tiles, blockIdx.x, r, b);
 #pragma unroll
     for (uint32_t k = 0; k < kOrderPer; ++k) atomicAdd(&s_bin[b[k]], 1u);
     __syncthreads();
@@ -717,12 +719,15 @@ __global__ void __launch_bounds__(kOrderThreads) k_tile_place(const __grid_const
     const uint32_t tiles = view.tiles;
     if (blockIdx.x * kOrderSlice >= tiles) return;
     const uint32_t* const slice_hist = view.slice_hist;
-    uint32_t *const order = view.order, *const status = view.status;
+    uint4* const order = view.order;
+    uint32_t* const status = &view.ctl->status;
     __shared__ uint32_t s_incl[64];
     __shared__ uint32_t s_base[64];
     const uint32_t tid = threadIdx.x, slices = (tiles + kOrderSlice - 1u) / kOrderSlice;
+    uint2 r[kOrderPer];
     uint32_t b[kOrderPer];
-    slice_bins(ranges, tiles, blockIdx.x, b);  // in flight while the table is summed
+    slice_bins(ranges, tiles, blockIdx.x, r, b);  // in flight while the table is summed
+    const uint32_t sorted = view.ctl->sorted_count;
     uint32_t total = 0, before = 0, incl = 0;
     if (tid < 64u) {  // warps 0 and 1: one bin per thread
         for (uint32_t s = 0; s < slices; ++s) {
@@ -746,9 +751,10 @@ __global__ void __launch_bounds__(kOrderThreads) k_tile_place(const __grid_const
         const uint32_t t = blockIdx.x * kOrderSlice + k * kOrderThreads + tid;
         if (t < tiles) {
             const uint32_t at = atomicAdd(&s_base[b[k]], 1u);
-            if (GS_IN_BOUNDS(at, tiles, status)) order[at] = t;
             // bin 63 is length 0: a tile the last sort pass left at its cleared bounds
-            if (b[k] == 63u) reinterpret_cast<uint2*>(ranges)[t] = make_uint2(0u, 0u);
+            if (b[k] == 63u) reinterpret_cast<uint2*>(ranges)[t] = r[k] = make_uint2(0u, 0u);
+            // a range past the sorted count can only come from a timed-out sort: clamp it
+            if (GS_IN_BOUNDS(at, tiles, status)) order[at] = make_uint4(t, r[k].x, min(r[k].y, sorted), 0u);
         }
     }
 }
@@ -795,7 +801,8 @@ void launch_frame_begin(FrameCtl* ctl, uint64_t* flags, uint32_t flag_words, cud
     launch_pdl(k_frame_begin, dim3(grid), dim3(256), s, ctl, ranges, range_words, flags, flag_words);
 }
 
-void launch_scan_emit(const EmitView* views, uint32_t count, uint32_t digit_bits, uint32_t slot, cudaStream_t s) {
+void launch_scan_emit(const EmitView* views, uint32_t count, uint32_t together, uint32_t digit_bits, uint32_t slot,
+                      cudaStream_t s) {
     uint32_t n = 0;
     for (uint32_t v = 0; v < count; ++v) n = std::max(n, views[v].n);
     auto launch = [&](auto kernel, auto kernel_views, uint32_t items) {
@@ -809,7 +816,8 @@ void launch_scan_emit(const EmitView* views, uint32_t count, uint32_t digit_bits
     // 512x512 13.8 / 13.2 / 15.7 / 28.5, a close-up of 60k 27.8 / 37.6 / 54 / 99, 100k at 320x240 14.5 / 13.6 /
     // 12.3 / 19.0, 250k in 8x8 tiles 31 / 26 / 24.7 / 32.4, 500k 44 / 30 / 17.8 / 19.8, 1M 80 / 49 / 28.9 / 30.8,
     // 3M at 4K - / - / 97 / 113, 8M - / - / 171 / 164, 16M - / - / 365 / 344
-    const uint64_t all = (uint64_t)n * count;  // several views fill the GPU together
+    // (the views of a batch fill the GPU together: 16 of 35k at 1080p 399 -> 396 us, 24 of 100k at 320x240 797 -> 791)
+    const uint64_t all = (uint64_t)n * together;
     if (all < 75000u) launch(k_scan_emit<1>, k_scan_emit_views<1>, 1u);
     else if (all < 150000u) launch(k_scan_emit<2>, k_scan_emit_views<2>, 2u);
     else if (n < 8000000u) launch(k_scan_emit<4>, k_scan_emit_views<4>, 4u);

@@ -106,7 +106,9 @@ struct EmitView {
     uint64_t* flags;
     uint32_t n, tiles_x, max_instance, passes;
 };
-void launch_scan_emit(const EmitView* views, uint32_t count, uint32_t digit_bits, uint32_t slot, cudaStream_t s);
+// together: the views whose launches run side by side, this one's included.
+void launch_scan_emit(const EmitView* views, uint32_t count, uint32_t together, uint32_t digit_bits, uint32_t slot,
+                      cudaStream_t s);
 
 // Onesweep LSD radix pass. n comes from *n_dev when non-null, else n_host. flags must hold
 // onesweep_flag_words(partitions, radix) words for the largest partition count the pass can see (the
@@ -155,7 +157,9 @@ void launch_exclusive_scan(uint32_t* data, uint32_t n, uint32_t* total_dev, Fram
 uint32_t tile_order_slices(uint32_t tiles);
 struct OrderView {
     uint32_t* ranges;
-    uint32_t *slice_hist, *order, *status;
+    uint32_t* slice_hist;
+    uint4* order;
+    FrameCtl* ctl;
     uint32_t tiles;
 };
 void launch_tile_order(const OrderView* views, uint32_t count, cudaStream_t s);
@@ -188,14 +192,12 @@ struct RasterOut {
 // leaves every tile ceil(length / 32) words of its own; a plane holds max_instance / 32 + tiles + 1.
 __host__ __device__ __forceinline__ size_t hit_mask_base(uint32_t start, uint32_t tile) { return (size_t)(start >> 5) + tile; }
 // configure_raster_kernels: kernel attributes, once per device. batch: a quarter of the range
-// positions culled per step (32 to 256). ctl (optional) bounds every range by the sorted count; n bounds the Gaussian indices; order
-// (optional) is the tile each CTA renders (launch_tile_order), else CTA i renders tile i.
+// positions staged per step (32 to 256). order: launch_tile_order's; n bounds the Gaussian indices.
 void configure_raster_kernels();
 struct RasterView {
-    const uint32_t *ranges, *vals;
+    const uint4* order;
+    const uint32_t* vals;
     const float4* rec;
-    const FrameCtl* ctl;
-    const uint32_t* order;
     RasterOut out;
     uint32_t n, width, height, tiles_x, tiles;
 };
@@ -222,11 +224,10 @@ cudaError_t static_scan_set_sequence(uint32_t seq);
 // float 8n on, dL/d(opacity). configure_raster_backward: kernel attributes, once per device.
 void configure_raster_backward();
 // hit_masks, mask_pitch: as the frame's forward raster left them (RasterOut).
-void launch_raster_backward(uint32_t tile, const uint32_t* ranges, const uint32_t* vals, const float4* rec, uint32_t n,
-                            const FrameCtl* ctl, uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
+void launch_raster_backward(uint32_t tile, const uint4* order, const uint32_t* vals, const float4* rec, uint32_t n,
+                            uint32_t width, uint32_t height, uint32_t tiles_x, uint32_t tiles_y,
                             const float* final_t, const uint32_t* n_contrib, const uint32_t* hit_masks,
-                            size_t mask_pitch, const float* dl_drgb, float* grad2d, const uint32_t* order,
-                            cudaStream_t s);
+                            size_t mask_pitch, const float* dl_drgb, float* grad2d, cudaStream_t s);
 // Up to kMaxMultiViews views of one scene for launch_preprocess_backward_multi.
 struct MultiViewGrads {
     const ViewBlock* view[kMaxMultiViews];

@@ -8,32 +8,40 @@
 //   testT = T * (1 - alpha);                                   done if testT < 1e-4
 //   C += colour * alpha * T (one fma per channel); T = testT
 //
-// Cull. The CTA takes the range in steps (4 x raster_batch positions, one vote per step to stop once every
-// pixel is done, raseter.wgsl:54-68): one lane per splat tests the octagon around the region where
+// Stage and cull. The CTA takes the range in steps (4 x raster_batch positions, at most 512, one vote per
+// step to stop once every pixel is done, raseter.wgsl:54-68): one lane per splat sends the record to shared
+// memory by asynchronous copies and meanwhile tests the octagon around the region where
 // power >= c_o = ln((1/255)/o) - 1e-3 can hold (its half extents come with the record,
 // gs_raster_common.cuh) against the CTA's blocks, and ballots turn the answers into one word per warp
 // and 32 positions. A splat outside a block would have been rejected by each of its pixels, so walking only
 // the hits changes no output bit. Contributor counts are range positions, so skipping does not change
 // them.
 //
-// Walk. From there a warp is on its own: it stages the records of its hits in a ring of its own by
-// asynchronous copies, 32 positions at a time, while it blends the hits staged before. A lane each lays
-// 16 to 32 hits out as pairs, and the arithmetic up to the blend (power, exp, alpha, 1 - alpha,
-// colour times alpha) runs on two splats at once by packed fp32 operations, which round each half like the
-// scalar ones; only the blend itself goes splat by splat, by predicated instructions. Below a power of -20
-// alpha is formed at -20, where every opacity's is under 1/255, so the cut-off need not travel with the hit.
+// Walk. From there a warp is on its own until the next step: it lists its hits, a lane each lays 32 of
+// them out as pairs, and the arithmetic up to the blend (power, exp, alpha, 1 - alpha, colour times alpha)
+// runs on two splats at once by packed fp32 operations, which round each half like the scalar ones; only
+// the blend itself goes splat by splat, by predicated instructions. Below a power of -20 alpha is formed at
+// -20, where every opacity's is under 1/255, so the cut-off need not travel with the hit.
 //
-// What bounds it: shared-memory reads of the hits' nine values (a 16-byte read returns 512 bytes to a
-// warp, four cycles of the SM's 128 bytes), 52% of the time at 1M / 1080p, the fp32 pipe 51%, issue 65%;
-// more warps (40 or 48 per SM, at 48 or 40 registers) measured the same, 24 slower. Measured against one CTA
-// per tile that staged 256 splats between two barriers, computed the octagon per tile and splat and walked
-// the bits of its ballots at one splat per step (32 registers, 2048 threads per SM): 1M / 1080p
-// 189.5 -> 181.8 us (216M -> 146M warp instructions), 3M / 4K 1168 -> 1031, 250k / 1237x823 in 8x8 tiles
-// 105 -> 72, a close-up of 60k at 1600x900 212 -> 187, 16 views in 32x32 tiles 3906 -> 2432 in sum, a 300-tile
-// view of 100k 76 -> 50, 50k / 512x512 47.6 -> 35.6. On the way, 1M / 1080p: the pairs alone 211 us
-// (3 selects per blend instead of predicates, octagons per tile, a barrier per 256 positions), predicates
-// and steps of 1024 200, without the cut-off's reads 195.5, half extents from the preprocess and up to 32 hits
-// per step 181.8; the packed constants read from constant memory 191.
+// What bounds it: where lists are long, shared-memory reads of the hits' nine values (a 16-byte read
+// returns 512 bytes to a warp, four cycles of the SM's 128 bytes), 49% of the time at 1M / 1080p, the fp32
+// pipe 50%, issue 65%; where they are short (a dozen splats a tile at 1080p) the chain of loads, tile, index,
+// record, that each CTA goes through. So the tile comes with its range (k_tile_place), a record is read once
+// per tile, and 40 warps fit an SM (46 to 48 registers, 34 KB per CTA; 48 of them at 8x8 tiles). Sixteen
+// sparse views of 35k at 1080p side by side: 338 us a batch, 368 with 32 warps, 332 with 48, which
+// cost 1M / 1080p 2%; steps of 256 cost it 2%, of 768 gain and lose nothing.
+//
+// Measured against one CTA per tile that staged 256 splats between two barriers, computed the octagon per
+// tile and splat and walked the bits of its ballots at one splat per step (32 registers, 2048 threads per
+// SM): 1M / 1080p 189.5 -> 178.3 us (216M -> 143M warp instructions), 3M / 4K 1168 -> 1024, 250k / 1237x823 in
+// 8x8 tiles 105 -> 75, a close-up of 60k at 1600x900 212 -> 182, 16 views in 32x32 tiles 3906 -> 2495 in
+// sum, 50k / 512x512 47.6 -> 42.7, the sixteen sparse views 341 -> 346. A ring of staged hits per warp, filled
+// from the record while the hits before are blended, between culling steps of 1024: 181.5, 1030, 72.4, 187,
+// 2445, 39.5 and 404 us; it read a record once per warp that it hits, and index and record twice in a row. On
+// the way to it, 1M / 1080p: the pairs alone 211 us (3 selects per blend instead of predicates, octagons per
+// tile, a barrier per 256 positions), predicates and steps of 1024 200, without the cut-off's reads 195.5, half
+// extents from the preprocess and up to 32 hits per step 181.8; the packed constants read from constant
+// memory 191.
 //
 // Tiles start in order[]'s order: by decreasing range length, so the longest tiles
 // start first instead of forming the tail of the launch (with tiles in index order the clustered
@@ -66,25 +74,29 @@ __device__ __forceinline__ uint32_t block_bits(float x, float y, const float4& e
     return e.x < __int_as_float(0x7f800000) ? bits : (1u << (WX * WY)) - 1u;
 }
 
-constexpr uint32_t kRing = 64;          // staged hits per warp (room for 32 more at kChunkMin + 16 pending)
-constexpr uint32_t kChunk = 32;         // most hits blended per step (one lane each lays them out in pairs)
-constexpr uint32_t kChunkMin = 16;      // fewest, until the tile's last
-constexpr uint32_t kMaxGroups = 32;     // groups of 32 range positions per cull step, at most
+constexpr uint32_t kChunk = 32;   // most hits blended at a time (one lane each lays them out in pairs)
+constexpr uint32_t kList = 64;    // hits waiting per warp (room for 32 more at kChunk - 1 pending)
 
-// Shared memory of a warp: a ring of staged hits and the step's hits as pairs.
+// Shared memory of a warp: its next hits (positions in the step) and the chunk's hits as pairs.
 struct RasterWarp {
-    float4 a[kRing];  // (x, y, conic.x, conic.y)
-    float4 b[kRing];  // (conic.z, opacity, r, g)
-    float4 c[kRing];  // (b, cut, range position, unused)
     float4 pair[kChunk / 2][5];  // (x, x', y, y'), (A, A', -B, -B'), (C, C', o, o'), (r, r', g, g'),
                                  // (b, b', position, position')
+    uint32_t list[kList];
 };
 template <int TILE>
 struct RasterShared {
     static constexpr int kSub = TILE < 16 ? TILE : 16;  // a CTA renders kSub x kSub pixels of a tile
     static constexpr int kWarps = kSub * kSub / 32;
+    // range positions per step, at most, and CTAs per SM: an 8x8 tile's two warps and short list leave no
+    // room for more of either (250k / 1237x823 with 128 positions and 48 warps 141 us a frame, 128 and 40
+    // 143, 256 and 32 145)
+    static constexpr uint32_t kStage = TILE < 16 ? 128 : 512;
+    static constexpr int kCtas = (TILE < 16 ? 48 : 40) / kWarps;
     RasterWarp warp[kWarps];
-    uint32_t masks[kMaxGroups][kWarps];  // the step's hits per group and warp
+    float4 a[kStage];  // the step's records: (x, y, conic.x, conic.y)
+    float4 b[kStage];  // (conic.z, opacity, r, g)
+    float2 c[kStage];  // (b, cut)
+    uint32_t masks[kStage / 32][kWarps];  // the step's hits per group of 32 positions and warp
 };
 
 // What a raster keeps besides the colours: nothing, the final transmittance, or that and the contributor
@@ -126,14 +138,30 @@ __device__ __forceinline__ void blend_one(float power, float alpha, float one_mi
 }
 #undef GS_BLEND
 
-// The CTA of sub-block `sub` of the tile at place `at` of the view's order.
+// One pixel's results.
+template <int KEEP>
+__device__ __forceinline__ void store_pixel(const RasterOut& out, size_t p, float cr, float cg, float cb, float final_t,
+                                            uint32_t last) {
+    if (out.rgb) {
+        out.rgb[3 * p + 0] = cr;
+        out.rgb[3 * p + 1] = cg;
+        out.rgb[3 * p + 2] = cb;
+    }
+    if (KEEP != kKeepNothing && out.final_t) out.final_t[p] = final_t;
+    if (KEEP == kKeepLast && out.n_contrib) out.n_contrib[p] = last;
+    if (out.rgba8) {
+        const uint32_t r8 = (uint32_t)(fminf(fmaxf(cr, 0.0f), 1.0f) * 255.0f + 0.5f);
+        const uint32_t g8 = (uint32_t)(fminf(fmaxf(cg, 0.0f), 1.0f) * 255.0f + 0.5f);
+        const uint32_t b8 = (uint32_t)(fminf(fmaxf(cb, 0.0f), 1.0f) * 255.0f + 0.5f);
+        out.rgba8[p] = r8 | (g8 << 8) | (b8 << 16) | (255u << 24);
+    }
+}
+
+// CTA `block` of a view: a sub-block of a tile, the longest tiles first.
 template <int TILE, int KEEP>
-__device__ __forceinline__ void raster_view(const RasterView& view, uint32_t at, uint32_t sub, uint32_t step) {
-    const uint32_t* __restrict__ const ranges = view.ranges;
+__device__ __forceinline__ void raster_view(const RasterView& view, uint32_t block, uint32_t step) {
     const uint32_t* __restrict__ const vals = view.vals;
     const float4* __restrict__ const rec = view.rec;
-    const FrameCtl* __restrict__ const ctl = view.ctl;
-    const uint32_t* __restrict__ const order = view.order;
     const RasterOut out = view.out;
     const uint32_t n = view.n, width = view.width, height = view.height, tiles_x = view.tiles_x;
     constexpr bool LAST = KEEP == kKeepLast;
@@ -142,40 +170,43 @@ __device__ __forceinline__ void raster_view(const RasterView& view, uint32_t at,
     extern __shared__ __align__(16) unsigned char s_raw[];
     RasterShared<TILE>& cta = *reinterpret_cast<RasterShared<TILE>*>(s_raw);
 
-    const uint32_t tile = order ? order[at] : at;
-    const uint32_t px0 = (tile % tiles_x) * TILE + kSub * (sub % kSubs), py0 = (tile / tiles_x) * TILE + kSub * (sub / kSubs);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint4 place = __ldg(view.order + block / (kSubs * kSubs));
+    const uint32_t tile = place.x, start = place.y, end = place.z, sub = block % (kSubs * kSubs);
+    const uint32_t px0 = (tile % tiles_x) * TILE + kSub * (sub % kSubs), py0 = (tile / tiles_x) * TILE + kSub * (sub / kSubs);
     RasterWarp& sh = cta.warp[warp];
     const uint32_t bx = 8u * (warp % (kSub / 8u)), by = 4u * (warp / (kSub / 8u));  // the warp's block
     const uint32_t x = px0 + bx + (lane & 7u), y = py0 + by + (lane >> 3);
     // plane of the hit masks: the block's number in the tile, row by row
     const uint32_t plane = ((kSub * (sub / kSubs) + by) / 4u) * (TILE / 8u) + (kSub * (sub % kSubs) + bx) / 8u;
     const bool inside = x < width && y < height;
-    const uint2 range = reinterpret_cast<const uint2*>(ranges)[tile];
-    // a range past the sorted count can only come from a timed-out sort: clamp it
-    const uint32_t end = ctl ? min(range.y, ctl->sorted_count) : range.y;
-    const uint32_t start = range.x;
     const float2 nfx = both(-(float)x), nfy = both(-(float)y);
 
     float T = inside ? 1.0f : 0.0f, final_t = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
     uint32_t last = 0;
-    uint32_t head = 0, ready = 0, tail = 0;  // hits blended, staged for certain, staged or on their way
+    uint32_t head = 0, tail = 0;             // hits blended, listed
     bool over = false;                       // every pixel of the warp is done
 
-    // blends the next cnt (at most kChunk) staged hits
-    auto blend = [&](uint32_t cnt) {
+    // blends the next cnt (at most kChunk) listed hits of the step whose first position is pos0
+    auto blend = [&](uint32_t cnt, uint32_t pos0) {
+        __syncwarp();  // the list
         {
-            const uint32_t slot = (head + lane) % kRing;
-            float4 a = sh.a[slot], b = sh.b[slot], c = sh.c[slot];
+            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+            float2 c = make_float2(0.0f, 0.0f);
             float* q = reinterpret_cast<float*>(sh.pair[lane >> 1]) + (lane & 1u);
-            // past the hits (where the ring may hold anything) alpha is 0; so it is below a positive
-            // cut-off, where the opacity itself is under 1/255
-            if (lane >= cnt) a = b = c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            // past the hits alpha is 0; so it is below a positive cut-off, where the opacity itself is under 1/255
+            uint32_t at = 0;
+            if (lane < cnt) {
+                at = sh.list[(head + lane) % kList];
+                a = cta.a[at];
+                b = cta.b[at];
+                c = cta.c[at];
+            }
             if (c.y > 0.0f) b.y = 0.0f;
             q[0] = a.x; q[2] = a.y; q[4] = a.z; q[6] = -a.w;
             q[8] = b.x; q[10] = b.y; q[12] = b.z; q[14] = b.w;
             q[16] = c.x;
-            if (LAST) q[18] = c.z;
+            if (LAST) q[18] = __uint_as_float(pos0 + at + 1u);
         }
         __syncwarp();
         const uint32_t pairs = (cnt + 1u) / 2u;
@@ -210,13 +241,18 @@ __device__ __forceinline__ void raster_view(const RasterView& view, uint32_t at,
     for (uint32_t i = start; i < end; i += step) {
         if (__syncthreads_and(over)) break;
         const uint32_t cnt = min(step, end - i);
-        // cull: each splat's octagon against the tile's blocks, one word per warp and 32 positions
+        // stage the records and cull: each splat's octagon against the tile's blocks, one word per warp and
+        // 32 positions
         for (uint32_t j = threadIdx.x; j < (cnt + 31u & ~31u); j += kThreads) {
             uint32_t bits = 0;
             const uint32_t g = j < cnt ? vals[i + j] : n;
             if (g < n) {  // always, unless the sort timed out
-                const float2 c = __ldg(reinterpret_cast<const float2*>(rec + (size_t)kRecFloat4 * g));
-                bits = block_bits<kSub>(c.x, c.y, __ldg(rec + (size_t)kRecFloat4 * g + 3), (float)px0, (float)py0);
+                const float4* r = rec + (size_t)kRecFloat4 * g;
+                cp_async16(&cta.a[j], r);
+                cp_async16(&cta.b[j], r + 1);
+                cp_async8(&cta.c[j], r + 2);
+                const float2 c = __ldg(reinterpret_cast<const float2*>(r));
+                bits = block_bits<kSub>(c.x, c.y, __ldg(r + 3), (float)px0, (float)py0);
             }
             uint32_t word = 0;
 #pragma unroll
@@ -226,83 +262,51 @@ __device__ __forceinline__ void raster_view(const RasterView& view, uint32_t at,
             }
             if (lane < kWarps) cta.masks[j >> 5][lane] = word;
         }
+        cp_async_commit();
+        cp_async_wait<0>();
         __syncthreads();
         if (over) continue;
         const uint32_t groups = (cnt + 31u) / 32u;
         const uint32_t words = lane < groups ? cta.masks[lane][warp] : 0u;
         if (LAST && lane < groups && out.hit_masks)  // the backward visits the same splats
             out.hit_masks[plane * out.mask_pitch + hit_mask_base(start, tile) + ((i - start) >> 5) + lane] = words;
-        uint32_t group = 0, m = 0, g = n;
-        // the next group with hits; its Gaussian indices are loaded while the group before it is staged
-        auto next_group = [&]() {
-            m = 0;
-            while (group < groups && (m = __shfl_sync(0xffffffffu, words, group)) == 0u) ++group;
-            if (m >> lane & 1u) g = vals[i + 32u * group + lane];
-        };
-        next_group();
-        while (m != 0u && !over) {
-            while (m != 0u && tail - head + __popc(m) <= kRing) {
-                if (m >> lane & 1u) {
-                    const uint32_t slot = (tail + __popc(m & ((1u << lane) - 1u))) % kRing;
-                    const float4* r = rec + (size_t)kRecFloat4 * g;
-                    cp_async16(&sh.a[slot], r);
-                    cp_async16(&sh.b[slot], r + 1);
-                    cp_async8(&sh.c[slot], r + 2);
-                    if (LAST) sh.c[slot].z = __uint_as_float(i - start + 32u * group + lane + 1u);
-                }
+        uint32_t any = __ballot_sync(0xffffffffu, words != 0u);
+        while (!over && (any != 0u || head < tail)) {
+            if (any != 0u && tail - head < kChunk) {
+                const uint32_t group = __ffs(any) - 1u, m = __shfl_sync(0xffffffffu, words, group);
+                if (m >> lane & 1u) sh.list[(tail + __popc(m & ((1u << lane) - 1u))) % kList] = 32u * group + lane;
                 tail += __popc(m);
-                ++group;
-                next_group();
+                any &= any - 1u;
+            } else {
+                blend(min(kChunk, tail - head), i - start);
             }
-            cp_async_commit();
-            cp_async_wait<1>();
-            __syncwarp();
-            if (ready - head >= kChunkMin) blend(min(kChunk, ready - head) & ~1u);
-            ready = tail;
         }
     }
-    cp_async_wait<0>();
-    __syncwarp();
-    while (head < tail && !over) blend(min(kChunk, tail - head));
-    if (!inside) return;
-    const size_t p = (size_t)y * width + x;
-    if (out.rgb) {
-        out.rgb[3 * p + 0] = cr;
-        out.rgb[3 * p + 1] = cg;
-        out.rgb[3 * p + 2] = cb;
-    }
-    if (KEEP != kKeepNothing && out.final_t) out.final_t[p] = final_t;
-    if (LAST && out.n_contrib) out.n_contrib[p] = last;
-    if (out.rgba8) {
-        const uint32_t r8 = (uint32_t)(fminf(fmaxf(cr, 0.0f), 1.0f) * 255.0f + 0.5f);
-        const uint32_t g8 = (uint32_t)(fminf(fmaxf(cg, 0.0f), 1.0f) * 255.0f + 0.5f);
-        const uint32_t b8 = (uint32_t)(fminf(fmaxf(cb, 0.0f), 1.0f) * 255.0f + 0.5f);
-        out.rgba8[p] = r8 | (g8 << 8) | (b8 << 16) | (255u << 24);
-    }
+    if (inside) store_pixel<KEEP>(out, (size_t)y * width + x, cr, cg, cb, final_t, last);
 }
 
 template <int TILE, int KEEP>
-__global__ void __launch_bounds__(RasterShared<TILE>::kWarps * 32, 32 / RasterShared<TILE>::kWarps)
+__global__ void __launch_bounds__(RasterShared<TILE>::kWarps * 32, RasterShared<TILE>::kCtas)
 k_raster(RasterView view, uint32_t step) {
     pdl_wait();
-    constexpr uint32_t kSubs = (TILE / RasterShared<TILE>::kSub) * (TILE / RasterShared<TILE>::kSub);
-    raster_view<TILE, KEEP>(view, blockIdx.x / kSubs, blockIdx.x % kSubs, step);
+    raster_view<TILE, KEEP>(view, blockIdx.x, step);
 }
 // Several views: their longest tiles first, view by view, then their next ones.
 template <int TILE, int KEEP>
-__global__ void __launch_bounds__(RasterShared<TILE>::kWarps * 32, 32 / RasterShared<TILE>::kWarps)
+__global__ void __launch_bounds__(RasterShared<TILE>::kWarps * 32, RasterShared<TILE>::kCtas)
 k_raster_views(const __grid_constant__ Views<RasterView> views, uint32_t step) {
     pdl_wait();
     constexpr uint32_t kSubs = (TILE / RasterShared<TILE>::kSub) * (TILE / RasterShared<TILE>::kSub);
     const uint32_t unit = blockIdx.x / kSubs, at = unit / views.count;
     const RasterView& view = views.view[unit % views.count];
     if (at >= view.tiles) return;
-    raster_view<TILE, KEEP>(view, at, blockIdx.x % kSubs, step);
+    raster_view<TILE, KEEP>(view, at * kSubs + blockIdx.x % kSubs, step);
 }
 
 template <int TILE>
 void launch_tile(const RasterView* views, uint32_t count, uint32_t step, cudaStream_t s) {
     constexpr uint32_t kSubs = TILE / RasterShared<TILE>::kSub;
+    step = std::min(step, RasterShared<TILE>::kStage);
     uint32_t tiles = 0;
     bool last = false, final_t = false;
     for (uint32_t v = 0; v < count; ++v) {
@@ -344,7 +348,7 @@ void configure_raster_kernels() {
 }
 
 void launch_raster(const RasterView* views, uint32_t count, uint32_t tile, uint32_t batch, cudaStream_t s) {
-    batch *= 4u;  // positions per cull step (128 to 1024, a multiple of 32): most tiles need one step
+    batch *= 4u;  // positions per step (a multiple of 32), as far as the stage goes: most tiles need one or two
     if (tile == 8) launch_tile<8>(views, count, batch, s);
     else if (tile == 32) launch_tile<32>(views, count, batch, s);
     else launch_tile<16>(views, count, batch, s);
