@@ -9,11 +9,10 @@
 //   C += colour * alpha * T (one fma per channel); T = testT
 //
 // Stage and cull. The CTA takes the range in steps (4 x raster_batch positions, at most 512, one vote per
-// step to stop once every pixel is done, raseter.wgsl:54-68): one lane per splat sends the record to shared
-// memory by asynchronous copies and meanwhile tests the octagon around the region where
-// power >= c_o = ln((1/255)/o) - 1e-3 can hold (its half extents come with the record,
-// gs_raster_common.cuh) against the CTA's blocks, and ballots turn the answers into one word per warp
-// and 32 positions. A splat outside a block would have been rejected by each of its pixels, so walking only
+// step to stop once every pixel is done, raseter.wgsl:54-68): one lane per splat tests the octagon around the
+// region where power >= c_o = ln((1/255)/o) - 1e-3 can hold (its half extents come with the record,
+// gs_raster_common.cuh) against the CTA's blocks, sends the record to shared memory by asynchronous copies
+// if it meets any, and ballots turn the answers into one word per warp and 32 positions. A splat outside a block would have been rejected by each of its pixels, so walking only
 // the hits changes no output bit. Contributor counts are range positions, so skipping does not change
 // them.
 //
@@ -24,24 +23,25 @@
 // -20, where every opacity's is under 1/255, so the cut-off need not travel with the hit.
 //
 // What bounds it: where lists are long, shared-memory reads of the hits' nine values (a 16-byte read
-// returns 512 bytes to a warp, four cycles of the SM's 128 bytes), 49% of the time at 1M / 1080p, the fp32
-// pipe 50%, issue 65%; where they are short (a dozen splats a tile at 1080p) the chain of loads, tile, index,
+// returns 512 bytes to a warp, four cycles of the SM's 128 bytes), 53% of the time at 1M / 1080p, the fp32
+// pipe 56%, issue 72%; where they are short (a dozen splats a tile at 1080p) the chain of loads, tile, index,
 // record, that each CTA goes through. So the tile comes with its range (k_tile_place), a record is read once
-// per tile, and 40 warps fit an SM (46 to 48 registers, 34 KB per CTA; 48 of them at 8x8 tiles). Sixteen
-// sparse views of 35k at 1080p side by side: 338 us a batch, 368 with 32 warps, 332 with 48, which
-// cost 1M / 1080p 2%; steps of 256 cost it 2%, of 768 gain and lose nothing.
+// per tile, and 40 warps fit an SM (46 to 48 registers, 34 KB per CTA; 48 of them at 8x8 tiles). With 32 / 40 / 48
+// warps: 1M / 1080p 306 / 299 / 310 us a frame, 12 views of 300k in 32x32 tiles 745 / 710 / 738, 16 sparse
+// views of 35k at 1080p 370 / 339 / 340; steps of 256 cost 1M / 1080p 2%, of 768 gain nothing.
 //
 // Measured against one CTA per tile that staged 256 splats between two barriers, computed the octagon per
 // tile and splat and walked the bits of its ballots at one splat per step (32 registers, 2048 threads per
-// SM): 1M / 1080p 189.5 -> 178.3 us (216M -> 143M warp instructions), 3M / 4K 1168 -> 1024, 250k / 1237x823 in
-// 8x8 tiles 105 -> 75, a close-up of 60k at 1600x900 212 -> 182, 16 views in 32x32 tiles 3906 -> 2495 in
-// sum, 50k / 512x512 47.6 -> 42.7, the sixteen sparse views 341 -> 346. A ring of staged hits per warp, filled
-// from the record while the hits before are blended, between culling steps of 1024: 181.5, 1030, 72.4, 187,
-// 2445, 39.5 and 404 us; it read a record once per warp that it hits, and index and record twice in a row. On
-// the way to it, 1M / 1080p: the pairs alone 211 us (3 selects per blend instead of predicates, octagons per
-// tile, a barrier per 256 positions), predicates and steps of 1024 200, without the cut-off's reads 195.5, half
-// extents from the preprocess and up to 32 hits per step 181.8; the packed constants read from constant
-// memory 191.
+// SM): 1M / 1080p 189.5 -> 162.4 us (216M -> 143M warp instructions), 3M / 4K 1168 -> 930, 250k / 1237x823 in
+// 8x8 tiles 105 -> 70, a close-up of 60k at 1600x900 212 -> 177, 16 views in 32x32 tiles 3906 -> 2198 in
+// sum, 50k / 512x512 47.6 -> 41.7, the sixteen sparse views 341 -> 344. Other ways to bring the records
+// in: all of a step's, hit or not, 178.3, 1024, 75.3, 182, 2495, 42.7 and 346 us (up to half of a list's splats meet
+// no block: the list is by the splat's bounding square); a ring of hits per warp, filled while the hits
+// before are blended, between culling steps of 1024, 181.5, 1030, 72.4, 187, 2445, 39.5 and 404 (a record is
+// read once per warp that it hits). On the way there, 1M / 1080p: the pairs alone 211 us (3 selects per
+// blend instead of predicates, octagons per tile, a barrier per 256 positions), predicates and steps of
+// 1024 200, without the cut-off's reads 195.5, half extents from the preprocess and up to 32 hits per step
+// 181.8; the packed constants read from constant memory 191.
 //
 // Tiles start in order[]'s order: by decreasing range length, so the longest tiles
 // start first instead of forming the tail of the launch (with tiles in index order the clustered
@@ -88,8 +88,8 @@ struct RasterShared {
     static constexpr int kSub = TILE < 16 ? TILE : 16;  // a CTA renders kSub x kSub pixels of a tile
     static constexpr int kWarps = kSub * kSub / 32;
     // range positions per step, at most, and CTAs per SM: an 8x8 tile's two warps and short list leave no
-    // room for more of either (250k / 1237x823 with 128 positions and 48 warps 141 us a frame, 128 and 40
-    // 143, 256 and 32 145)
+    // room for more of either (250k / 1237x823 with 128 positions and 48 warps 133 us a frame, 128 and 40
+    // 135, 256 and 32 135)
     static constexpr uint32_t kStage = TILE < 16 ? 128 : 512;
     static constexpr int kCtas = (TILE < 16 ? 48 : 40) / kWarps;
     RasterWarp warp[kWarps];
@@ -248,11 +248,13 @@ __device__ __forceinline__ void raster_view(const RasterView& view, uint32_t blo
             const uint32_t g = j < cnt ? vals[i + j] : n;
             if (g < n) {  // always, unless the sort timed out
                 const float4* r = rec + (size_t)kRecFloat4 * g;
-                cp_async16(&cta.a[j], r);
-                cp_async16(&cta.b[j], r + 1);
-                cp_async8(&cta.c[j], r + 2);
                 const float2 c = __ldg(reinterpret_cast<const float2*>(r));
                 bits = block_bits<kSub>(c.x, c.y, __ldg(r + 3), (float)px0, (float)py0);
+                if (bits) {
+                    cp_async16(&cta.a[j], r);
+                    cp_async16(&cta.b[j], r + 1);
+                    cp_async8(&cta.c[j], r + 2);
+                }
             }
             uint32_t word = 0;
 #pragma unroll
