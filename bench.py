@@ -121,32 +121,33 @@ def algorithmic_bytes(fi: dict, n: int, pixels: int, passes: int) -> dict:
         # the tile ranges cleared, the control block's counters and digit histograms reset
         "frame begin": 8 * tiles + 8 * 1024,
         # 12 B position of every Gaussian + the other 224 B of each one in front of the near plane;
-        # writes: 4 B count each, 48 B raster record per near-plane survivor, 16 B rect per visible
-        "preprocess": 12 * n + 224 * npass + 4 * n + 48 * npass + 16 * vis,
+        # writes: 4 B count each, 64 B raster record per near-plane survivor, 16 B rect per visible
+        "preprocess": 12 * n + 224 * npass + 4 * n + 64 * npass + 16 * vis,
         # counts + rects in, offsets + keys/values out
         "scan+emit": 4 * (n + 1) + 16 * vis + 4 * (n + 1) + 8 * s,
         # each pass reads and writes keys and values (the last one also leaves the tile ranges)
         "sort": passes * 16 * s,
-        # the ranges read twice (bin counts, placement), the order written
-        "tile order": 2 * 8 * tiles + 4 * tiles,
-        # per instance the index and the 48 B record, per tile its range, per pixel 4 B rgba8
-        "raster": 52 * s + 8 * tiles + 4 * pixels,
+        # the ranges read twice (bin counts, placement), the order written with them
+        "tile order": 2 * 8 * tiles + 16 * tiles,
+        # per instance the index and the 64 B record, per tile its place and range, per pixel 4 B rgba8
+        "raster": 68 * s + 16 * tiles + 4 * pixels,
     }
 
 
 # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum, one ncu --set full capture of
 # the forward frame of this workload on a GB300) and what bounds each kernel there.
-NCU_TRAFFIC_BYTES = {"preprocess": 286.5e6, "raster": 56.6e6}
+NCU_TRAFFIC_BYTES = {"preprocess": 307.8e6, "raster": 61.0e6}
 # issue-slot utilisation of the kernels bound by instruction issue (ncu smsp__issue_active, one
 # capture of the kernel at this workload): for them this, not the HBM fraction, is the efficiency measure
-NCU_ISSUE_ACTIVE = {"raster": 0.933}
+NCU_ISSUE_ACTIVE = {"raster": 0.737}
 # warp instructions per launch (ncu smsp__inst_executed.sum, the same capture): the numerator of the
 # issue-rate roofline of those kernels (four issue slots per SM per cycle)
-NCU_WARP_INSTRUCTIONS = {"raster": 275.27e6}
+NCU_WARP_INSTRUCTIONS = {"raster": 180.27e6}
 LIMITER = {
-    "raster": "instruction issue (ncu: issue slots busy 93.3% at full residency, DRAM 3% of peak; the "
-              "48-byte records are re-read from L2, so DRAM traffic is below the algorithmic bytes)",
-    "preprocess": "HBM and the pinned arithmetic (ncu: 69% of DRAM peak, 70% of issue slots)",
+    "raster": "instruction issue, the fp32 pipe and shared-memory reads together (ncu: issue slots busy 73.7%, "
+              "fp32 pipe 59%, shared-memory data 55%, DRAM 4% of peak; the 64-byte records are re-read from L2, so "
+              "DRAM traffic is below the algorithmic bytes)",
+    "preprocess": "HBM and the pinned arithmetic (ncu: 70% of issue slots)",
 }
 
 

@@ -12,9 +12,9 @@
 // step to stop once every pixel is done, raseter.wgsl:54-68): one lane per splat tests the octagon around the
 // region where power >= c_o = ln((1/255)/o) - 1e-3 can hold (its half extents come with the record,
 // gs_raster_common.cuh) against the CTA's blocks, sends the record to shared memory by asynchronous copies
-// if it meets any, and ballots turn the answers into one word per warp and 32 positions. A splat outside a block would have been rejected by each of its pixels, so walking only
-// the hits changes no output bit. Contributor counts are range positions, so skipping does not change
-// them.
+// if it meets any, and ballots turn the answers into one word per warp and 32 positions. A splat outside a
+// block would have been rejected by each of its pixels, so walking only the hits changes no output bit.
+// Contributor counts are range positions, so skipping does not change them.
 //
 // Walk. From there a warp is on its own until the next step: it lists its hits, a lane each lays 32 of
 // them out as pairs, and the arithmetic up to the blend (power, exp, alpha, 1 - alpha, colour times alpha)
@@ -35,8 +35,8 @@
 // SM): 1M / 1080p 189.5 -> 162.4 us (216M -> 143M warp instructions), 3M / 4K 1168 -> 930, 250k / 1237x823 in
 // 8x8 tiles 105 -> 70, a close-up of 60k at 1600x900 212 -> 177, 16 views in 32x32 tiles 3906 -> 2198 in
 // sum, 50k / 512x512 47.6 -> 41.7, the sixteen sparse views 341 -> 344. Other ways to bring the records
-// in: all of a step's, hit or not, 178.3, 1024, 75.3, 182, 2495, 42.7 and 346 us (up to half of a list's splats meet
-// no block: the list is by the splat's bounding square); a ring of hits per warp, filled while the hits
+// in: all of a step's, hit or not, 178.3, 1024, 75.3, 182, 2495, 42.7 and 346 us (a list takes its splats by their
+// bounding squares, so many of them meet no block); a ring of hits per warp, filled while the hits
 // before are blended, between culling steps of 1024, 181.5, 1030, 72.4, 187, 2445, 39.5 and 404 (a record is
 // read once per warp that it hits). On the way there, 1M / 1080p: the pairs alone 211 us (3 selects per
 // blend instead of predicates, octagons per tile, a barrier per 256 positions), predicates and steps of
