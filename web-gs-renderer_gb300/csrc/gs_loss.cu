@@ -9,6 +9,13 @@
 //   k_ssim_bwd  blurred partials + the L1 term -> dL/dx.
 // Images are H x W x 3 (pixel-interleaved). The loss is not bit-pinned: this file is built with
 // multiply-add contraction and the approximate division, and its filters use fused multiply-adds.
+//
+// What bounds it: instruction issue (about 80% of slots), of which the filters' multiply-adds are under
+// half. So the staging spends as little as it can on addresses: a warp takes whole rows, with one comparison
+// and one 32-bit offset for all images, instead of a division by the tile's edge per element (66.2M -> 60.1M
+// warp instructions forward, 50.5M -> 40.6M backward at 1080p). Both kernels a call: 1080p 122.7 -> 110.0
+// us, 720p 55.8 -> 49.0, 397x301 12.5 -> 11.1, 4K 506 -> 455. Four CTAs per SM and 64 registers: with five (48) 120.9, with
+// three (72) 118.4.
 #include <cmath>
 
 #include "gs_kernels.h"
@@ -31,31 +38,59 @@ constexpr int kItemsH = kH * (kT / kRunH);  // 168 row runs
 constexpr int kRunV = 4;            // vertical pass: 4 consecutive outputs of one column per thread
 static_assert(kT * (kT / kRunV) == kThreads, "one vertical run per thread");
 
-// Stages rows [ty0, ty0 + kH) x cols [tx0, tx0 + kH) of channel ch of an H x W x 3 image (zeros
-// outside) into dst (pitch kPitchIn).
-__device__ __forceinline__ void stage_channel(const float* __restrict__ img, uint32_t W, uint32_t H, int tx0,
-                                              int ty0, int ch, float* dst) {
-    // a fixed trip count, so that all of a thread's loads are in flight before the first store
-    constexpr int kIters = (kH * kH + kThreads - 1) / kThreads;
-    float v[kIters];
+// Stages rows [ty0, ty0 + kH) x cols [tx0, tx0 + kH) of N images (src: pixel (0, 0); elements `pixel` apart
+// along a row, `row` from row to row; zeros outside) into dst (pitch kPitchIn). A warp takes every eighth
+// row, a lane one of its first 32 columns, so that a row costs one addition and one comparison; the last 10
+// columns are dealt out singly. Fixed trip counts, so that all of a thread's loads are in flight before the
+// first store.
+template <int N>
+__device__ __forceinline__ void stage(const float* const (&src)[N], uint32_t pixel, uint32_t row, uint32_t W, uint32_t H,
+                                      int tx0, int ty0, float* const (&dst)[N]) {
+    constexpr int kWarps = kThreads / 32, kRows = (kH + kWarps - 1) / kWarps;
+    constexpr int kTail = kH - 32, kTails = (kH * kTail + kThreads - 1) / kThreads;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int gx = tx0 + lane, gy0 = ty0 + warp;
+    const bool col = (uint32_t)gx < W;
+    float v[kRows][N], t[kTails][N];
+    // offsets from the tile's corner fit 32 bits (42 rows)
+    const ptrdiff_t corner = (ptrdiff_t)ty0 * (ptrdiff_t)row + (ptrdiff_t)tx0 * (ptrdiff_t)pixel;
+    const float* base[N];
 #pragma unroll
-    for (int it = 0; it < kIters; ++it) {
-        const int i = threadIdx.x + it * kThreads;
-        const int ly = i / kH, lx = i - ly * kH, gx = tx0 + lx, gy = ty0 + ly;
-        v[it] = 0.0f;
-        if (i < kH * kH && gx >= 0 && gx < (int)W && gy >= 0 && gy < (int)H) v[it] = img[((size_t)gy * W + gx) * 3 + ch];
+    for (int q = 0; q < N; ++q) base[q] = src[q] + corner;
+    const uint32_t first = warp * row + lane * pixel;
+#pragma unroll
+    for (int k = 0; k < kRows; ++k) {
+        const bool in = col && (uint32_t)(gy0 + kWarps * k) < H && warp + kWarps * k < kH;
+        const uint32_t o = first + kWarps * k * row;
+#pragma unroll
+        for (int q = 0; q < N; ++q) v[k][q] = in ? base[q][o] : 0.0f;
     }
 #pragma unroll
-    for (int it = 0; it < kIters; ++it) {
-        const int i = threadIdx.x + it * kThreads;
-        if (i < kH * kH) dst[(i / kH) * kPitchIn + i % kH] = v[it];
+    for (int k = 0; k < kTails; ++k) {
+        const int i = threadIdx.x + k * kThreads, ly = i / kTail, lx = 32 + i % kTail;
+        const bool in = i < kH * kTail && (uint32_t)(tx0 + lx) < W && (uint32_t)(ty0 + ly) < H;
+        const uint32_t o = ly * row + lx * pixel;
+#pragma unroll
+        for (int q = 0; q < N; ++q) t[k][q] = in ? base[q][o] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < kRows; ++k)
+        if (warp + kWarps * k < kH)
+#pragma unroll
+            for (int q = 0; q < N; ++q) dst[q][(warp + kWarps * k) * kPitchIn + lane] = v[k][q];
+#pragma unroll
+    for (int k = 0; k < kTails; ++k) {
+        const int i = threadIdx.x + k * kThreads;
+        if (i < kH * kTail)
+#pragma unroll
+            for (int q = 0; q < N; ++q) dst[q][(i / kTail) * kPitchIn + 32 + i % kTail] = t[k][q];
     }
 }
 
 // Moments of x and y over the window, the SSIM map, its partials with respect to the moments, and
 // per-block sums of SSIM and |x - y|. Each thread filters a run of 8 outputs of one row (the 18 inputs
 // it needs stay in registers), then a run of 4 outputs of one column.
-__global__ void __launch_bounds__(kThreads) k_ssim_fwd(const float* __restrict__ x, const float* __restrict__ y,
+__global__ void __launch_bounds__(kThreads, 4) k_ssim_fwd(const float* __restrict__ x, const float* __restrict__ y,
                                                        uint32_t W, uint32_t H, Window win,
                                                        float* __restrict__ partial /* 9 planes */,
                                                        double* __restrict__ block_sums) {
@@ -66,8 +101,11 @@ __global__ void __launch_bounds__(kThreads) k_ssim_fwd(const float* __restrict__
     const int ch = blockIdx.z;
     const int tx0 = blockIdx.x * kT - kR, ty0 = blockIdx.y * kT - kR;
     const int tid = threadIdx.x;
-    stage_channel(x, W, H, tx0, ty0, ch, sx);
-    stage_channel(y, W, H, tx0, ty0, ch, sy);
+    {
+        const float* const src[2] = {x + ch, y + ch};
+        float* const dst[2] = {sx, sy};
+        stage(src, 3, 3 * W, W, H, tx0, ty0, dst);
+    }
     __syncthreads();
     if (tid < kItemsH) {
         const int r = tid / (kT / kRunH), c0 = (tid % (kT / kRunH)) * kRunH;
@@ -114,6 +152,8 @@ __global__ void __launch_bounds__(kThreads) k_ssim_fwd(const float* __restrict__
             for (int k = 0; k < 2 * kR + 1; ++k) m[o][q] = fmaf(win.w[k], v[o + k], m[o][q]);
     }
     const size_t P = (size_t)W * H;
+    float* const first = partial + (size_t)(ch * 3) * P + (size_t)(blockIdx.y * kT + r0) * W + gx;
+    float* const out[3] = {first, first + P, first + 2 * P};
     float ssim = 0.0f, l1 = 0.0f;
 #pragma unroll
     for (int o = 0; o < kRunV; ++o) {
@@ -129,10 +169,9 @@ __global__ void __launch_bounds__(kThreads) k_ssim_fwd(const float* __restrict__
         const float ds_dmx = (2.0f * my * A2) * inv_b - sv * (2.0f * mx) * (B2 * inv_b);
         const float ds_dsxx = -sv * (B1 * inv_b);
         const float ds_dsxy = 2.0f * A1 * inv_b;
-        const size_t po = (size_t)gy * W + gx;
-        partial[(ch * 3 + 0) * P + po] = ds_dmx + ds_dsxx * (-2.0f * mx) + ds_dsxy * (-my);
-        partial[(ch * 3 + 1) * P + po] = ds_dsxx;
-        partial[(ch * 3 + 2) * P + po] = ds_dsxy;
+        out[0][o * W] = ds_dmx + ds_dsxx * (-2.0f * mx) + ds_dsxy * (-my);
+        out[1][o * W] = ds_dsxx;
+        out[2][o * W] = ds_dsxy;
         ssim += sv;
         l1 += fabsf(sx[(r0 + o + kR) * kPitchIn + c + kR] - sy[(r0 + o + kR) * kPitchIn + c + kR]);
     }
@@ -163,7 +202,7 @@ __device__ void reduce_sums(double* __restrict__ sums, size_t blocks);
 
 // sums (may be null): block 0 also reduces the forward's per-block sums into sums[0..1], while the
 // other blocks filter, so the loss value needs no kernel of its own when a gradient is formed.
-__global__ void __launch_bounds__(kThreads) k_ssim_bwd(const float* __restrict__ partial, const float* __restrict__ x,
+__global__ void __launch_bounds__(kThreads, 4) k_ssim_bwd(const float* __restrict__ partial, const float* __restrict__ x,
                                                        const float* __restrict__ y, uint32_t W, uint32_t H,
                                                        Window win, float lambda, float* __restrict__ dl,
                                                        double* __restrict__ sums, size_t sum_blocks) {
@@ -177,35 +216,21 @@ __global__ void __launch_bounds__(kThreads) k_ssim_bwd(const float* __restrict__
     const size_t P = (size_t)W * H;
     const int c = tid % kT, r0 = (tid / kT) * kRunV;
     const int gx = blockIdx.x * kT + c;
+    const size_t at = ((size_t)(blockIdx.y * kT + r0) * W + gx) * 3 + ch;  // the thread's first output
     // this thread's x and y, loaded first so that they arrive during the staging and the filtering
     float xv[kRunV], yv[kRunV];
 #pragma unroll
     for (int o = 0; o < kRunV; ++o) {
         const int gy = blockIdx.y * kT + r0 + o;
         const bool in = gx < (int)W && gy < (int)H;
-        const size_t q = in ? ((size_t)gy * W + gx) * 3 + ch : 0;
-        xv[o] = in ? x[q] : 0.0f;
-        yv[o] = in ? y[q] : 0.0f;
+        xv[o] = in ? x[at + 3 * W * o] : 0.0f;
+        yv[o] = in ? y[at + 3 * W * o] : 0.0f;
     }
     {
-        constexpr int kIters = (kH * kH + kThreads - 1) / kThreads;
-        float v[kIters][3];
-#pragma unroll
-        for (int it = 0; it < kIters; ++it) {
-            const int i = tid + it * kThreads;
-            const int ly = i / kH, lx = i - ly * kH, gx = tx0 + lx, gy = ty0 + ly;
-            const bool in = i < kH * kH && gx >= 0 && gx < (int)W && gy >= 0 && gy < (int)H;
-            const size_t o = in ? (size_t)gy * W + gx : 0;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) v[it][q] = in ? partial[(ch * 3 + q) * P + o] : 0.0f;
-        }
-#pragma unroll
-        for (int it = 0; it < kIters; ++it) {
-            const int i = tid + it * kThreads;
-            if (i < kH * kH)
-#pragma unroll
-                for (int q = 0; q < 3; ++q) sp[q][(i / kH) * kPitchIn + i % kH] = v[it][q];
-        }
+        const float* const src[3] = {partial + (size_t)(ch * 3) * P, partial + (size_t)(ch * 3 + 1) * P,
+                                     partial + (size_t)(ch * 3 + 2) * P};
+        float* const dst[3] = {sp[0], sp[1], sp[2]};
+        stage(src, 1, W, W, H, tx0, ty0, dst);
     }
     __syncthreads();
     if (tid < kItemsH) {
@@ -244,10 +269,9 @@ __global__ void __launch_bounds__(kThreads) k_ssim_bwd(const float* __restrict__
     for (int o = 0; o < kRunV; ++o) {
         const int gy = blockIdx.y * kT + r0 + o;
         if (gx >= (int)W || gy >= (int)H) continue;
-        const size_t q = ((size_t)gy * W + gx) * 3 + ch;
         const float d = xv[o] - yv[o];
         const float g_l1 = (d > 0.0f ? inv : (d < 0.0f ? -inv : 0.0f));
-        dl[q] = g_l1 - lambda * inv * (bl[o][0] + 2.0f * xv[o] * bl[o][1] + yv[o] * bl[o][2]);
+        dl[at + 3 * W * o] = g_l1 - lambda * inv * (bl[o][0] + 2.0f * xv[o] * bl[o][1] + yv[o] * bl[o][2]);
     }
 }
 
