@@ -192,7 +192,7 @@ struct RasterOut {
 // leaves every tile ceil(length / 32) words of its own; a plane holds max_instance / 32 + tiles + 1.
 __host__ __device__ __forceinline__ size_t hit_mask_base(uint32_t start, uint32_t tile) { return (size_t)(start >> 5) + tile; }
 // configure_raster_kernels: kernel attributes, once per device. batch: a quarter of the range
-// positions staged per step (32 to 256). order: launch_tile_order's; n bounds the Gaussian indices.
+// positions staged per step (32 to 256; a step is 512 at most, 128 in 8x8 tiles). order: launch_tile_order's; n bounds the Gaussian indices.
 void configure_raster_kernels();
 struct RasterView {
     const uint4* order;
