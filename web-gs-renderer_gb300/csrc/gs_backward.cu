@@ -96,7 +96,7 @@ __device__ __forceinline__ void pix_load(PixState& p, uint32_t x, uint32_t y, ui
 // dC/dalpha_i = T_i c_i - S_i / (1 - alpha_i), S_i being the colour added behind splat i, so
 // dL/dalpha_i = T_i K_i - D_i / (1 - alpha_i) with K_i = dC . c_i and D_i = dC . S_i, and D grows by
 // alpha_i T_i K_i per step. No branch on the rejections: a rejected pixel takes alpha = 0 and K = 0, which
-// leaves its state as it is and gives two zeros.
+// leaves its state as it is, and gives two zeros, also where D is no longer finite.
 __device__ __forceinline__ void pix_step(PixState& p, uint32_t pos, const float4& a, const float4& b,
                                          const float2& c, float& gp, float& w) {
     const float dx = a.x - p.fx, dy = a.y - p.fy;
@@ -113,7 +113,7 @@ __device__ __forceinline__ void pix_step(PixState& p, uint32_t pos, const float4
     p.T = p.T * ria;  // transmittance in front of this splat
     w = alpha * p.T;
     const float dalpha = __fmaf_rn(p.T, k, -(p.d * ria));
-    gp = og <= kAlphaClamp ? dalpha * alpha : 0.0f;  // a clamped alpha passes no gradient
+    gp = in & (og <= kAlphaClamp) ? dalpha * alpha : 0.0f;  // a clamped alpha passes no gradient
     p.d = __fmaf_rn(w, k, p.d);
 }
 
@@ -139,7 +139,7 @@ __device__ __forceinline__ void pix_step2(PixState& p, const float4& p0, const f
         p.T = p.T * ria;
         w = alpha * p.T;
         const float dalpha = __fmaf_rn(p.T, k, -(p.d * ria));
-        gp = og <= kAlphaClamp ? dalpha * alpha : 0.0f;
+        gp = in & (og <= kAlphaClamp) ? dalpha * alpha : 0.0f;
         p.d = __fmaf_rn(w, k, p.d);
     };
     one(power.x, og.x, kk.x, __float_as_uint(p4.z), gp.x, w.x);
