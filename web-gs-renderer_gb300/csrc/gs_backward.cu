@@ -4,8 +4,8 @@
 //                         visited (its hit masks) back to front from the block's last contributor,
 //                         recomputing power and alpha bit for bit as the forward did (same pinned
 //                         arithmetic), recovering T by division, and accumulating dL/d(pixel.xy, conic,
-//                         opacity, colour) per Gaussian: eight hits at a time reduced over the block's
-//                         pixels by matrix instructions, three vector atomics per hit. Up to the pixel's own
+//                         opacity, colour) per Gaussian: eight hits at a time summed over the block's
+//                         pixels, four lanes to a hit, two vector atomics and a scalar one per hit. Up to the pixel's own
 //                         chain the arithmetic runs on two hits at once by packed fp32 operations.
 // The preprocess half (2D gradients -> the 59 attributes) is in gs_preprocess_backward.cu.
 // Conventions: gradients flow through the fp32 RGB before quantization; culled Gaussians, skipped
@@ -18,31 +18,20 @@
 namespace gs {
 namespace {
 
-// ---- reduction of a hit's gradients on the tensor cores --------------------------------------------
-// With P_k(u, v) = {1, u, v, u^2, uv, v^2} over the pixel's offset (u, v) from its block's centre and
-// gp = dL/dpower of a (pixel, splat) pair, w = alpha T its blending weight, the nine gradients of a splat
-// over a warp's pixels follow from nine sums: the six moments sum(gp P_k) (dx = X - u and dy = Y - v are
-// affine in the pixel, so the sums of gp dx^i dy^j are polynomials in the splat's X, Y with the moments as
-// coefficients; dL/do is the zeroth over o) and the three sum(w dC). That is a matrix product of the
-// hits' [gp; w] rows with fixed columns: a pixel adds two values per hit instead of accumulating nine,
-// and eight hits at a time are reduced by mma.sync m16n8k8 (tf32, fp32 accumulators): rows 0-7 the hits'
-// gp, rows 8-15 their w, k the warp's pixels, columns either P_k (small multiples of 1/4: exact in tf32)
-// or dC split into its tf32 head and tail. gp and w are split into head and tail too (an mma reads the
-// upper 19 bits of an operand), so a product keeps 22 bits and more, and the accumulators are fp32.
+// ---- reduction of a hit's gradients over a block --------------------------------------------------------
+// Of a (pixel, splat) pair there are gp = dL/dpower and w = alpha T, its blending weight; the splat's nine
+// gradients follow from nine sums over the block's pixels: gp, gp dx, gp dy, gp dx^2, gp dx dy, gp dy^2 and w dC
+// (dL/do is the first over o). The pixels leave gp and w of eight hits in shared memory and each hit is then
+// summed by four lanes, a row of eight pixels each (dy is the row's), so that a pixel adds two values per hit
+// instead of nine and the lanes meet in ten shuffles per eight hits.
+//
+// All of it is fp32, and dx and dy are the splat's own: sums of gp times powers of the pixel's offset from the
+// block's centre, moved to the splat afterwards, cancel where the splat is narrow (at X from the centre of
+// the block by X^2 over the mean dx^2), and as products on tf32 matrix instructions, operands split in two
+// halves, they keep 22 bits. That form was here before: the scales' gradients of splats about a pixel wide
+// were 9.1e-7 off 64 bits instead of 5.8e-7 (colours of splats of two pixels 4.0e-7 instead of 3.4e-7), and it was slower
+// (1M / 1080p 283 us, now 260).
 constexpr uint32_t kHits = 8;  // hits per flush
-
-__device__ __forceinline__ void mma_tf32(float d[4], const float a[4], float b0, float b1, const float c[4]) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
-          "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
-}
-
-// tf32 head of v, rounded to nearest (two integer operations; cvt.rna.tf32.f32 takes four here); v minus it
-// is exact and serves as the second operand, of which the mma drops at most the last bit.
-__device__ __forceinline__ float tf32_head(float v) {
-    return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u);
-}
 
 // Predicated adds to global memory (no branch around them).
 __device__ __forceinline__ void red_add4_if(bool on, float* p, float x, float y, float z, float w) {
@@ -150,7 +139,7 @@ __device__ __forceinline__ bool pix_finite(const PixState& p) {
     return finite_f(p.dr) && finite_f(p.dg) && finite_f(p.db);
 }
 
-// A pixel whose dL/dC is not finite stays out of the matrix products (a zero weight times it would be
+// A pixel whose dL/dC is not finite stays out of the block sums (a zero weight times it would be
 // NaN in every hit of its warp): it walks its part of the tile's list by itself and adds its gradients
 // one by one.
 __device__ __noinline__ void walk_alone(PixState p, const uint32_t* __restrict__ vals, uint32_t len,
@@ -177,21 +166,20 @@ __device__ __noinline__ void walk_alone(PixState p, const uint32_t* __restrict__
     }
 }
 
-constexpr uint32_t kRowUnits = 20;  // 16-byte units per row: 16 pixel pairs, padded so that the eight
-                                    // lanes that read two rows at once hit distinct banks
+constexpr uint32_t kRowPitch = 36;  // floats per row: 32 pixels, padded so that the eight lanes that read
+                                    // two rows at once hit distinct banks
 constexpr uint32_t kRing = 64;      // staged hits per warp (room for 32 more at two flushes' pending)
 constexpr uint32_t kChunk = 32;     // most hits laid out in pairs at once
 constexpr uint32_t kBwdWarps = 2;   // warps per CTA; they share nothing
 
-// Shared memory of a warp: a ring of staged hits and the rows of kHits of them. A unit of a row holds two
-// neighbouring lanes' (gp, w): the mma's k and k + 4.
+// Shared memory of a warp: a ring of staged hits, and what the pixels add to kHits of them.
 struct BwdWarp {
     float4 a[kRing];  // (x, y, conic.x, conic.y)
     float4 b[kRing];  // (conic.z, opacity, r, g)
     float4 c[kRing];  // (b, cut, range position, Gaussian)
     float4 pair[kChunk / 2][5];  // (x, x', y, y'), (A, A', -B, -B'), (C, C', o, o'), (r, r', g, g'),
                                  // (b, b', position, position')
-    float4 rows[kHits * kRowUnits];
+    float gp[kHits][kRowPitch], w[kHits][kRowPitch];
 };
 
 // One warp per 8x4 block, one lane per pixel, no barrier between warps. The forward left one word per
@@ -202,14 +190,11 @@ struct BwdWarp {
 // batches, computed the cull again and met at two barriers per batch, a hit's bookkeeping (finding the
 // next bit, addresses, the counter of the pending rows) is gone.
 //
-// Bound by instruction issue (73% of slots at 28 warps per SM) and shared-memory reads (67%) where the
-// blocks fill the GPU, by the longest list otherwise. Measured against a CTA per tile with shuffle
-// reductions and two pixels per lane, mixture scenes: 1M / 1080p 405 -> 284 us (427M -> 250M warp
-// instructions); 3M / 1080p 879 -> 584; 500k / 720p (a list of 2300 splats) 358 -> 141; 20k / 397x301 92 -> 24. On
-// the way, 1M / 1080p in thousand cycles, from 839: matrix sums but a CTA per tile, 8x8 blocks with two pixels
-// per lane 1008, 8x4 blocks 847; 8x4 blocks by the hit masks 693; the chain's divide as one reciprocal and no
-// branch in a hit 664; columns without selects and predicated atomics 631; heads by integer rounding 603;
-// hits in pairs on packed operations 577, their loop fully unrolled 560.
+// Bound by instruction issue and shared-memory reads where the blocks fill the GPU, by the longest list otherwise. Measured against a CTA per tile with shuffle
+// reductions and two pixels per lane, mixture scenes: 1M / 1080p 405 -> 260 us; 500k / 720p (a list of 2300 splats)
+// 358 -> 129; 20k / 397x301 92 -> 24. On the way, with the block's sums on matrix instructions (above), 1M /
+// 1080p in thousand cycles, from 839: the chain's divide as one reciprocal and no branch in a hit 693 -> 664;
+// predicated atomics 631; hits in pairs on packed operations 577, their loop fully unrolled 560.
 template <int TILE>
 __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backward(const uint4* __restrict__ order,
                                                                      const uint32_t* __restrict__ vals,
@@ -224,7 +209,6 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
                                                                      float* __restrict__ grad2d) {
     pdl_wait();
     constexpr uint32_t WX = TILE / 8, kTileWarps = TILE * TILE / 32;
-    constexpr float kCx = 3.5f, kCy = 1.5f;  // centre of a warp's block
     __shared__ BwdWarp s_warp[kBwdWarps];
     BwdWarp& sh = s_warp[threadIdx.x >> 5];
 
@@ -247,37 +231,25 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
     }
     const uint32_t wmax = min(__reduce_max_sync(0xffffffffu, p.L), len);
     if (wmax == 0u) return;
-    // this lane's part of the columns: column fr at the pixels of lanes 2 m and 2 m + 1, m = 4 i + fc, for
-    // step i of the product (offsets u = 2 fc + h - 3.5 and v = i - 1.5); the colour columns are r, g, b
-    // heads, one unused, r, g, b tails, one unused
+    // of a flush a lane sums hit fr over row fc of the block: the row's dL/dC, in pairs of pixels
     const uint32_t fr = lane >> 2, fc = lane & 3u;
-    float poly[4][2], colour[4][2];
+    float2 dr[4], dg[4], db[4];
     {
-        // P_k as a product of two of 1, u, v: 11, u1, v1, uu, uv, vv
-        const float f0 = fr == 0u ? 1.0f : 0.0f, fu = fr == 1u || fr == 3u || fr == 4u ? 1.0f : 0.0f, fv = 1.0f - f0 - fu;
-        const float g0 = fr < 3u ? 1.0f : 0.0f, gu = fr == 3u ? 1.0f : 0.0f, gv = 1.0f - g0 - gu;
-        float* const plane = reinterpret_cast<float*>(sh.rows);
+        float* const plane = sh.gp[0];
         plane[lane] = p.dr;
         plane[32u + lane] = p.dg;
         plane[64u + lane] = p.db;
-        plane[96u + lane] = 0.0f;
         __syncwarp();
+        const float2* const row = reinterpret_cast<const float2*>(plane) + 4u * fc;
 #pragma unroll
-        for (uint32_t i = 0; i < 4u; ++i) {
-            const float v = (float)i - kCy;
-            const float2 d2 = reinterpret_cast<const float2*>(plane)[16u * (fr & 3u) + 4u * i + fc];
-            const float d[2] = {d2.x, d2.y};
-#pragma unroll
-            for (uint32_t h = 0; h < 2u; ++h) {
-                const float u = (float)(2u * fc + h) - kCx;
-                poly[i][h] = (f0 + fu * u + fv * v) * (g0 + gu * u + gv * v);  // exact
-                const float head = tf32_head(d[h]);
-                colour[i][h] = fr < 4u ? head : d[h] - head;
-            }
+        for (uint32_t k = 0; k < 4u; ++k) {
+            dr[k] = row[k];
+            dg[k] = row[16u + k];
+            db[k] = row[32u + k];
         }
         __syncwarp();
     }
-    const float cx = (float)bx0 + kCx, cy = (float)by0 + kCy;
+    const float row_x = (float)bx0, row_y = (float)(by0 + fc);
 
     // lays the next cnt (at most kChunk) staged hits out as pairs, a lane each
     auto lay_out = [&](uint32_t h0, uint32_t cnt) {
@@ -302,40 +274,61 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
             const float4* r = sh.pair[4u * v + u];
             float2 gp, w;
             pix_step2(p, r[0], r[1], r[2], r[3], r[4], gp, w);
-            float2* row = reinterpret_cast<float2*>(sh.rows) + 4u * kRowUnits * u + lane;
-            row[0] = make_float2(gp.x, w.x);
-            row[2u * kRowUnits] = make_float2(gp.y, w.y);
+            sh.gp[2u * u][lane] = gp.x;
+            sh.gp[2u * u + 1u][lane] = gp.y;
+            sh.w[2u * u][lane] = w.x;
+            sh.w[2u * u + 1u][lane] = w.y;
         }
         __syncwarp();
-        float m[4] = {0.0f, 0.0f, 0.0f, 0.0f}, q[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-        for (uint32_t i = 0; i < 4u; ++i) {
-            const float4 v = sh.rows[fr * kRowUnits + 4u * i + fc];
-            const float head[4] = {tf32_head(v.x), tf32_head(v.y), tf32_head(v.z), tf32_head(v.w)};
-            const float tail[4] = {v.x - head[0], v.y - head[1], v.z - head[2], v.w - head[3]};
-            mma_tf32(m, head, poly[i][0], poly[i][1], m);
-            mma_tf32(q, head, colour[i][0], colour[i][1], q);
-            mma_tf32(m, tail, poly[i][0], poly[i][1], m);
-            mma_tf32(q, tail, colour[i][0], colour[i][1], q);
-        }
-        // m[0..1]: moments 2 fc, 2 fc + 1 of hit fr; q[2..3]: colour columns 2 fc, 2 fc + 1
-        const float s0 = __shfl_sync(0xffffffffu, m[0], 0, 4), su = __shfl_sync(0xffffffffu, m[1], 0, 4);
-        const float sv = __shfl_sync(0xffffffffu, m[0], 1, 4), suu = __shfl_sync(0xffffffffu, m[1], 1, 4);
-        const float suv = __shfl_sync(0xffffffffu, m[0], 2, 4), svv = __shfl_sync(0xffffffffu, m[1], 2, 4);
-        const float c0 = q[2] + __shfl_xor_sync(0xffffffffu, q[2], 2);  // r (fc 0), b (fc 1)
-        const float c1 = q[3] + __shfl_xor_sync(0xffffffffu, q[3], 2);  // g (fc 0)
         const uint32_t slot = (h0 + fr) % kRing;
         const float4 a = sh.a[slot];
         const float2 b = *reinterpret_cast<const float2*>(&sh.b[slot]);
         const uint32_t gi = __float_as_uint(sh.c[slot].w);
-        const float X = a.x - cx, Y = a.y - cy;
-        const float sx = __fmaf_rn(X, s0, -su), sy = __fmaf_rn(Y, s0, -sv);  // sums of gp dx, gp dy
-        const float sxx = __fmaf_rn(X, sx - su, suu), syy = __fmaf_rn(Y, sy - sv, svv);
-        const float sxy = __fmaf_rn(Y, sx, __fmaf_rn(-X, sv, suv));
-        const bool first = fc == 0u, valid = fr < cnt && gi < n;
-        red_add4_if(valid && fc < 2u, grad2d + (size_t)8 * gi + 4u * fc, first ? -__fmaf_rn(a.z, sx, a.w * sy) : -0.5f * sxx,
-                    first ? -__fmaf_rn(b.x, sy, a.w * sx) : -sxy, first ? c0 : -0.5f * syy, first ? c1 : c0);
-        red_add_if(valid && fc == 2u && s0 != 0.0f, grad2d + (size_t)8 * n + gi, s0 * fast_rcp(b.y));
+        const float4 g0 = *reinterpret_cast<const float4*>(&sh.gp[fr][8u * fc]);
+        const float4 g1 = *reinterpret_cast<const float4*>(&sh.gp[fr][8u * fc + 4u]);
+        const float4 w0 = *reinterpret_cast<const float4*>(&sh.w[fr][8u * fc]);
+        const float4 w1 = *reinterpret_cast<const float4*>(&sh.w[fr][8u * fc + 4u]);
+        const float2 g[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
+        const float2 wt[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w), make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+        const float x0 = a.x - row_x, dy = a.y - row_y;
+        float2 dx = make_float2(x0, x0 - 1.0f);
+        float2 t = __fmul2_rn(g[0], dx), s0 = g[0], sx = t, sxx = __fmul2_rn(t, dx);
+        float2 r = __fmul2_rn(wt[0], dr[0]), gr = __fmul2_rn(wt[0], dg[0]), bl = __fmul2_rn(wt[0], db[0]);
+#pragma unroll
+        for (uint32_t k = 1; k < 4u; ++k) {
+            dx = __fadd2_rn(dx, both(-2.0f));
+            t = __fmul2_rn(g[k], dx);
+            s0 = __fadd2_rn(s0, g[k]);
+            sx = __fadd2_rn(sx, t);
+            sxx = __ffma2_rn(t, dx, sxx);
+            r = __ffma2_rn(wt[k], dr[k], r);
+            gr = __ffma2_rn(wt[k], dg[k], gr);
+            bl = __ffma2_rn(wt[k], db[k], bl);
+        }
+        // sums over the row: gp, gp dx, gp dy, gp dx^2, gp dx dy, gp dy^2, w dC
+        float sum0 = s0.x + s0.y;
+        const float rx = sx.x + sx.y, ry = dy * sum0;
+        const float even[4] = {rx, ry, r.x + r.y, gr.x + gr.y};
+        const float odd[4] = {sxx.x + sxx.y, dy * rx, dy * ry, bl.x + bl.y};
+        // and over the four rows: the even lanes of a hit get the first four, the odd ones the others
+        const bool first = (fc & 1u) == 0u;
+        float v4[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k) {
+            v4[k] = (first ? even[k] : odd[k]) + __shfl_xor_sync(0xffffffffu, first ? odd[k] : even[k], 1);
+            v4[k] += __shfl_xor_sync(0xffffffffu, v4[k], 2);
+        }
+        sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1);
+        sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
+        const bool valid = fr < cnt && gi < n;
+        // four zeros (no pixel of the block blended the splat) are not added: times a conic that is not finite they
+        // would be NaN
+        const bool some = ((__float_as_uint(v4[0]) | __float_as_uint(v4[1]) | __float_as_uint(v4[2]) | __float_as_uint(v4[3])) << 1) != 0u;
+        red_add4_if(valid && some && fc < 2u, grad2d + (size_t)8 * gi + 4u * fc,
+                    first ? -__fmaf_rn(a.z, v4[0], a.w * v4[1]) : -0.5f * v4[0],
+                    first ? -__fmaf_rn(b.x, v4[1], a.w * v4[0]) : -v4[1], first ? v4[2] : -0.5f * v4[2], v4[3]);
+        const float ro = fast_rcp(b.y);  // and a Newton step: 1 / o, nearly rounded
+        red_add_if(valid && fc == 2u && sum0 != 0.0f, grad2d + (size_t)8 * n + gi, sum0 * __fmaf_rn(ro, __fmaf_rn(-b.y, ro, 1.0f), ro));
         __syncwarp();
     };
 
