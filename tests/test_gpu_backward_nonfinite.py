@@ -46,3 +46,22 @@ def test_a_gaussian_without_a_finite_colour(tile, bad):
         at += width
         assert np.isfinite(g).all(), width
         assert np.abs(g - ref).max() <= 1e-5 * np.abs(ref).max(), width
+
+
+def test_no_finite_gradient_anywhere_costs_no_more_than_a_finite_one():
+    """A diverged step (dL/drgb all NaN) takes the walk that every other step takes. Measured 1.0 times the finite
+    step's time; pixels that walk their lists one by one take ten times as long, so the bound is 3."""
+    spec, cam = W.SceneSpec(300_000, 2, 1, 64, 20.0), W.CAMERA_720P
+    dl = np.random.default_rng(8).normal(0.0, 1e-3, (cam.height, cam.width, 3)).astype(np.float32)
+    ms = []
+    with webgs.Context(flags=webgs.GS_FLAG_DIFFERENTIABLE | webgs.GS_FLAG_PROFILE) as ctx:
+        sc = ctx.upload(spec.build(), spec.count)
+        for d in (dl, np.full_like(dl, np.nan)):
+            times = []
+            for _ in range(5):
+                ctx.forward(sc, cam.view(), rgba8=False, rgb=True)
+                ctx.backward(sc, d)
+                times.append(ctx.timings()["raster backward"]["ms"])
+            ms.append(min(times))
+        sc.close()
+    assert ms[1] <= 3.0 * ms[0], ms

@@ -30,7 +30,7 @@ namespace {
 // the block by X^2 over the mean dx^2), and as products on tf32 matrix instructions, operands split in two
 // halves, they keep 22 bits. That form was here before: the scales' gradients of splats about a pixel wide
 // were 9.1e-7 off 64 bits instead of 5.8e-7 (colours of splats of two pixels 4.0e-7 instead of 3.4e-7), and it was slower
-// (1M / 1080p 283 us, now 260).
+// (1M / 1080p 283 us, then 260).
 constexpr uint32_t kHits = 8;  // hits per flush
 
 // Predicated adds to global memory (no branch around them).
@@ -78,38 +78,17 @@ __device__ __forceinline__ void pix_load(PixState& p, uint32_t x, uint32_t y, ui
     }
 }
 
-// Visits the splat at 1-based range position pos for one pixel: the same power / exp / alpha
-// decisions as the forward (bit for bit); gp = dL/dpower and its blending weight w, zeros if the pixel
-// did not blend it. T is recovered by division (the approximate reciprocal, 1 ulp, of 1 - alpha >= 0.01 is
+// Visits two splats for one pixel, the one at the higher position first (back to front): the same power / exp /
+// alpha decisions as the forward (bit for bit); gp = dL/dpower and the blending weight w of each, zeros where the
+// pixel did not blend it. T is recovered by division (the approximate reciprocal, 1 ulp, of 1 - alpha >= 0.01 is
 // accurate enough for a gradient). With C = sum_i alpha_i T_i c_i and T_{i+1} = T_i (1 - alpha_i),
 // dC/dalpha_i = T_i c_i - S_i / (1 - alpha_i), S_i being the colour added behind splat i, so
 // dL/dalpha_i = T_i K_i - D_i / (1 - alpha_i) with K_i = dC . c_i and D_i = dC . S_i, and D grows by
 // alpha_i T_i K_i per step. No branch on the rejections: a rejected pixel takes alpha = 0 and K = 0, which
-// leaves its state as it is, and gives two zeros, also where D is no longer finite.
-__device__ __forceinline__ void pix_step(PixState& p, uint32_t pos, const float4& a, const float4& b,
-                                         const float2& c, float& gp, float& w) {
-    const float dx = a.x - p.fx, dy = a.y - p.fy;
-    const float power = __fmaf_rn(-0.5f, __fmaf_rn(a.z * dx, dx, (b.x * dy) * dy), -((a.w * dx) * dy));
-    const float og = raster_alpha_unclamped(b.y, power);  // the forward's o * exp(power)
-    float alpha = fminf(kAlphaClamp, og);
-    // from here on only gradients are formed: fused multiply-adds are fine (the decisions
-    // follow the forward's pinned arithmetic)
-    float k = __fmaf_rn(b.z, p.dr, __fmaf_rn(b.w, p.dg, c.x * p.db));  // dC . c
-    const bool in = (pos <= p.L) & !(power > 0.0f) & !(power < c.y) & (alpha >= kEpsilon);
-    alpha = in ? alpha : 0.0f;
-    k = in ? k : 0.0f;
-    const float ria = fast_rcp(1.0f - alpha);
-    p.T = p.T * ria;  // transmittance in front of this splat
-    w = alpha * p.T;
-    const float dalpha = __fmaf_rn(p.T, k, -(p.d * ria));
-    gp = in & (og <= kAlphaClamp) ? dalpha * alpha : 0.0f;  // a clamped alpha passes no gradient
-    p.d = __fmaf_rn(w, k, p.d);
-}
-
-// The same for two splats, the one at the higher position first (back to front): what does not depend on the
-// pixel's state is formed for both at once by packed operations (each half rounds like the scalar form).
+// leaves its state as it is, and gives two zeros, also where D is no longer finite. What does not depend on the
+// pixel's state is formed for both splats at once by packed operations (each half rounds like the scalar form).
 // Pairs as the walk lays them out; opacity 0 stands for one below every cut-off (its alpha is 0).
-__device__ __forceinline__ void pix_step2(PixState& p, const float4& p0, const float4& p1, const float4& p2,
+__device__ __forceinline__ void pix_step(PixState& p, const float4& p0, const float4& p1, const float4& p2,
                                           const float4& p3, const float4& p4, float2& gp, float2& w) {
     const float2 dx = __fadd2_rn(make_float2(p0.x, p0.y), both(-p.fx)), dy = __fadd2_rn(make_float2(p0.z, p0.w), both(-p.fy));
     const float2 q = __ffma2_rn(__fmul2_rn(make_float2(p1.x, p1.y), dx), dx,
@@ -133,37 +112,6 @@ __device__ __forceinline__ void pix_step2(PixState& p, const float4& p0, const f
     };
     one(power.x, og.x, kk.x, __float_as_uint(p4.z), gp.x, w.x);
     one(power.y, og.y, kk.y, __float_as_uint(p4.w), gp.y, w.y);
-}
-
-__device__ __forceinline__ bool pix_finite(const PixState& p) {
-    return finite_f(p.dr) && finite_f(p.dg) && finite_f(p.db);
-}
-
-// A pixel whose dL/dC is not finite stays out of the block sums (a zero weight times it would be
-// NaN in every hit of its warp): it walks its part of the tile's list by itself and adds its gradients
-// one by one.
-__device__ __noinline__ void walk_alone(PixState p, const uint32_t* __restrict__ vals, uint32_t len,
-                                        const float4* __restrict__ rec, uint32_t n, float* __restrict__ grad2d) {
-    for (uint32_t pos = min(p.L, len); pos > 0u; --pos) {
-        const uint32_t gi = vals[pos - 1u];
-        if (gi >= n) continue;
-        const float4 a = rec[(size_t)kRecFloat4 * gi], b = rec[(size_t)kRecFloat4 * gi + 1];
-        const float4 r2 = rec[(size_t)kRecFloat4 * gi + 2];
-        float gp, w;
-        pix_step(p, pos, a, b, make_float2(r2.x, r2.y), gp, w);
-        if (w == 0.0f) continue;  // not blended (a blended pair's weight is positive)
-        const float dx = a.x - p.fx, dy = a.y - p.fy;
-        float* q = grad2d + (size_t)8 * gi;
-        atomicAdd(q + 0, -gp * (a.z * dx + a.w * dy));
-        atomicAdd(q + 1, -gp * (b.x * dy + a.w * dx));
-        atomicAdd(q + 2, w * p.dr);
-        atomicAdd(q + 3, w * p.dg);
-        atomicAdd(q + 4, -0.5f * gp * dx * dx);
-        atomicAdd(q + 5, -gp * dx * dy);
-        atomicAdd(q + 6, -0.5f * gp * dy * dy);
-        atomicAdd(q + 7, w * p.db);
-        atomicAdd(grad2d + (size_t)8 * n + gi, gp / b.y);
-    }
 }
 
 constexpr uint32_t kRowPitch = 36;  // floats per row: 32 pixels, padded so that the eight lanes that read
@@ -224,13 +172,9 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
 
     PixState p;
     pix_load(p, bx0 + (lane & 7u), by0 + (lane >> 3), width, height, final_t, n_contrib, dl_drgb);
-    if (!pix_finite(p)) {
-        walk_alone(p, vals + start, len, rec, n, grad2d);
-        p.L = 0;
-        p.dr = p.dg = p.db = 0.0f;
-    }
     const uint32_t wmax = min(__reduce_max_sync(0xffffffffu, p.L), len);
     if (wmax == 0u) return;
+    const bool all_finite = __all_sync(0xffffffffu, finite_f(p.dr) && finite_f(p.dg) && finite_f(p.db));
     // of a flush a lane sums hit fr over row fc of the block: the row's dL/dC, in pairs of pixels
     const uint32_t fr = lane >> 2, fc = lane & 3u;
     float2 dr[4], dg[4], db[4];
@@ -273,7 +217,7 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
         for (uint32_t u = 0; u < kHits / 2u; ++u) {
             const float4* r = sh.pair[4u * v + u];
             float2 gp, w;
-            pix_step2(p, r[0], r[1], r[2], r[3], r[4], gp, w);
+            pix_step(p, r[0], r[1], r[2], r[3], r[4], gp, w);
             sh.gp[2u * u][lane] = gp.x;
             sh.gp[2u * u + 1u][lane] = gp.y;
             sh.w[2u * u][lane] = w.x;
@@ -293,7 +237,6 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
         const float x0 = a.x - row_x, dy = a.y - row_y;
         float2 dx = make_float2(x0, x0 - 1.0f);
         float2 t = __fmul2_rn(g[0], dx), s0 = g[0], sx = t, sxx = __fmul2_rn(t, dx);
-        float2 r = __fmul2_rn(wt[0], dr[0]), gr = __fmul2_rn(wt[0], dg[0]), bl = __fmul2_rn(wt[0], db[0]);
 #pragma unroll
         for (uint32_t k = 1; k < 4u; ++k) {
             dx = __fadd2_rn(dx, both(-2.0f));
@@ -301,15 +244,32 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
             s0 = __fadd2_rn(s0, g[k]);
             sx = __fadd2_rn(sx, t);
             sxx = __ffma2_rn(t, dx, sxx);
-            r = __ffma2_rn(wt[k], dr[k], r);
-            gr = __ffma2_rn(wt[k], dg[k], gr);
-            bl = __ffma2_rn(wt[k], db[k], bl);
         }
+        auto weighted = [&](const float2 (&d)[4]) {
+            float2 v = __fmul2_rn(wt[0], d[0]);
+#pragma unroll
+            for (uint32_t k = 1; k < 4u; ++k) v = __ffma2_rn(wt[k], d[k], v);
+            return v.x + v.y;
+        };
+        // a pixel whose dL/dC is not finite must not reach the splats that it does not blend: zero times it
+        // would be NaN (a blended pair's weight is positive). A whole image of NaN at 1M / 1080p takes 0.376 ms
+        // (a finite one 0.338, and 4.9 where such pixels walked their tile's list one by one).
+        auto weighted_blended = [&](const float2 (&d)[4]) {
+            float v = 0.0f;
+#pragma unroll
+            for (uint32_t k = 0; k < 4u; ++k) {
+                v += wt[k].x != 0.0f ? wt[k].x * d[k].x : 0.0f;
+                v += wt[k].y != 0.0f ? wt[k].y * d[k].y : 0.0f;
+            }
+            return v;
+        };
+        const float red = all_finite ? weighted(dr) : weighted_blended(dr), green = all_finite ? weighted(dg) : weighted_blended(dg);
+        const float blue = all_finite ? weighted(db) : weighted_blended(db);
         // sums over the row: gp, gp dx, gp dy, gp dx^2, gp dx dy, gp dy^2, w dC
         float sum0 = s0.x + s0.y;
         const float rx = sx.x + sx.y, ry = dy * sum0;
-        const float even[4] = {rx, ry, r.x + r.y, gr.x + gr.y};
-        const float odd[4] = {sxx.x + sxx.y, dy * rx, dy * ry, bl.x + bl.y};
+        const float even[4] = {rx, ry, red, green};
+        const float odd[4] = {sxx.x + sxx.y, dy * rx, dy * ry, blue};
         // and over the four rows: the even lanes of a hit get the first four, the odd ones the others
         const bool first = (fc & 1u) == 0u;
         float v4[4];
