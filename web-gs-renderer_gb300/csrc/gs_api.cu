@@ -96,8 +96,7 @@ struct Frame {
     DevBuf<uint4> order;  // tiles and ranges by decreasing length: the raster CTAs' tile order
     DevBuf<uint32_t> order_hist;  // per-slice bin counts of the tile order (64 words per 1024 tiles)
     DevBuf<uint32_t> rgba8, n_contrib;
-    DevBuf<uint32_t> hit_masks;  // differentiable frames: the raster's hits per 8x4 block (RasterOut)
-    size_t mask_pitch = 0;
+    size_t mask_pitch = 0;  // of the last frame's hit masks
     DevBuf<float> rgb, final_t;
     DevBuf<float> grad2d, dl_stage;
     bool grad2d_zero = false;  // grad2d holds zeros (cleared by the last preprocess backward)
@@ -107,6 +106,10 @@ struct Frame {
     uint32_t n = 0, width = 0, height = 0, tiles_x = 0, tiles_y = 0, passes = 0, max_instance = 0;
     int sorted_buf = 0;
     bool valid = false;
+    // a differentiable frame's raster leaves its hits per 8x4 block (RasterOut) where the sort's last pass took its
+    // values from: nothing reads those any more, and the masks' planes (64 bytes per Gaussian at 16x16 tiles, 256
+    // at 32x32) need no memory of their own
+    uint32_t* hit_masks() const { return vals[sorted_buf ^ 1].p; }
     bool direct_rgba8 = false, direct_rgb = false;  // the raster writes the caller's host buffer itself
 
     cudaError_t init(cudaStream_t s) {
@@ -120,13 +123,13 @@ struct Frame {
         ctl.pads(l); view.pads(l); rec.pads(l); meta.pads(l); counts.pads(l); offsets.pads(l);
         for (int b = 0; b < 2; ++b) { keys[b].pads(l); vals[b].pads(l); }
         flags.pads(l); ranges.pads(l); order.pads(l); order_hist.pads(l); rgba8.pads(l); n_contrib.pads(l);
-        hit_masks.pads(l); rgb.pads(l); final_t.pads(l); grad2d.pads(l); dl_stage.pads(l);
+        rgb.pads(l); final_t.pads(l); grad2d.pads(l); dl_stage.pads(l);
     }
     void release() {
         ctl.release(); view.release(); rec.release(); meta.release(); counts.release(); offsets.release();
         for (int b = 0; b < 2; ++b) { keys[b].release(); vals[b].release(); }
         flags.release(); ranges.release(); rgba8.release(); n_contrib.release(); rgb.release(); final_t.release();
-        order.release(); order_hist.release(); hit_masks.release(); grad2d.release(); dl_stage.release();
+        order.release(); order_hist.release(); grad2d.release(); dl_stage.release();
         if (h_ctl) cudaFreeHost(h_ctl);
         h_ctl = nullptr;
     }
@@ -137,7 +140,7 @@ struct FrameArgs {
     const gs_scene* scene;
     const ViewBlock* view;  // device copy of the view block
     uint32_t n, w, h, tiles_x, tiles_y, passes, max_instance;
-    size_t mask_pitch;  // words per plane of the frame's hit masks
+    size_t mask_pitch, mask_words;  // words per plane of a differentiable frame's hit masks, and of all planes
     RasterOut out;
 };
 
@@ -269,6 +272,7 @@ int frame_args(gs_ctx* ctx, const gs_scene* scene, const gs_view* view, FrameArg
     a->tiles_y = tiles_y;
     a->max_instance = scene->n * ctx->cfg.max_instance_factor;
     a->mask_pitch = (size_t)a->max_instance / 32 + (size_t)tiles + 1;
+    a->mask_words = a->mask_pitch * (tile * tile / 32);
     const uint32_t key_bits = 16u + bitlen((uint32_t)tiles - 1u);
     a->passes = (key_bits + ctx->cfg.digit_bits - 1) / ctx->cfg.digit_bits;
     return GS_OK;
@@ -279,14 +283,15 @@ int ensure_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a) {
     const uint32_t radix = 1u << ctx->cfg.digit_bits;
     const void* before[] = {f.rec.p, f.meta.p, f.counts.p, f.offsets.p, f.keys[0].p, f.keys[1].p, f.vals[0].p,
                             f.vals[1].p, f.flags.p, f.ranges.p, f.rgba8.p, f.rgb.p, f.final_t.p, f.n_contrib.p,
-                            f.order.p, f.order_hist.p, f.hit_masks.p};
+                            f.order.p, f.order_hist.p};
     GS_CK(f.rec.reserve((size_t)a.n * kRecFloat4));
     GS_CK(f.meta.reserve(a.n));
     GS_CK(f.counts.reserve(((size_t)a.n + 1 + 7) / 8 * 8));
     GS_CK(f.offsets.reserve((size_t)a.n + 1));
     for (int b = 0; b < 2; ++b) {
         GS_CK(f.keys[b].reserve(a.max_instance));
-        GS_CK(f.vals[b].reserve(a.max_instance));
+        const bool masks = (ctx->cfg.flags & GS_FLAG_DIFFERENTIABLE) && b == (int)((a.passes & 1u) ^ 1u);
+        GS_CK(f.vals[b].reserve(masks ? std::max<size_t>(a.max_instance, a.mask_words) : a.max_instance));
     }
     const size_t sort_parts = ((size_t)a.max_instance + ctx->cfg.sort_block - 1) / ctx->cfg.sort_block;
     const size_t scan_parts = ((size_t)a.n + 1 + kEmitPartitionMin - 1) / kEmitPartitionMin;
@@ -303,11 +308,9 @@ int ensure_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a) {
     GS_CK(f.rgb.reserve(pix * 3));
     GS_CK(f.final_t.reserve(pix));
     GS_CK(f.n_contrib.reserve(pix));
-    if (ctx->cfg.flags & GS_FLAG_DIFFERENTIABLE)
-        GS_CK(f.hit_masks.reserve(a.mask_pitch * (ctx->cfg.tile_size * ctx->cfg.tile_size / 32)));
     const void* after[] = {f.rec.p, f.meta.p, f.counts.p, f.offsets.p, f.keys[0].p, f.keys[1].p, f.vals[0].p,
                            f.vals[1].p, f.flags.p, f.ranges.p, f.rgba8.p, f.rgb.p, f.final_t.p, f.n_contrib.p,
-                           f.order.p, f.order_hist.p, f.hit_masks.p};
+                           f.order.p, f.order_hist.p};
     if (std::memcmp(before, after, sizeof(before)) != 0) ++ctx->alloc_gen;
     return GS_OK;
 }
@@ -325,7 +328,7 @@ void* mapped_host(const void* p) {
     return attr.type == cudaMemoryTypeHost ? attr.devicePointer : nullptr;
 }
 
-RasterOut raster_out(const gs_ctx* ctx, Frame& f, const gs_image* out, size_t mask_pitch) {
+RasterOut raster_out(const gs_ctx* ctx, Frame& f, const gs_image* out, const FrameArgs& a) {
     const bool dev = out && out->location == GS_MEM_DEVICE;
     const bool keep = (ctx->cfg.flags & GS_FLAG_DIFFERENTIABLE) != 0;
     RasterOut ro{};
@@ -344,8 +347,8 @@ RasterOut raster_out(const gs_ctx* ctx, Frame& f, const gs_image* out, size_t ma
     if (keep) {
         ro.final_t = f.final_t.p;
         ro.n_contrib = f.n_contrib.p;
-        ro.hit_masks = f.hit_masks.p;
-        ro.mask_pitch = mask_pitch;
+        ro.hit_masks = f.vals[(a.passes & 1u) ^ 1u].p;  // Frame::hit_masks once the frame is remembered
+        ro.mask_pitch = a.mask_pitch;
     } else if (out) {
         ro.final_t = out->final_t ? (dev ? out->final_t : f.final_t.p) : nullptr;
         ro.n_contrib = out->n_contrib ? (dev ? out->n_contrib : f.n_contrib.p) : nullptr;
@@ -755,7 +758,7 @@ int gs_forward(gs_ctx* ctx, const gs_scene* scene, const gs_view* view, const gs
     rc = ensure_frame(ctx, f, a);
     if (rc != GS_OK) return rc;
     a.view = f.view.p;
-    a.out = raster_out(ctx, f, out, a.mask_pitch);
+    a.out = raster_out(ctx, f, out, a);
     {
         const uint32_t slot = ctx->next_slot;
         ctx->next_slot = (slot + 1) % kViewSlots;
@@ -850,7 +853,7 @@ static int forward_batch(gs_ctx* ctx, const gs_batch_view* views, uint32_t count
     }
     for (uint32_t i = 0; i < count; ++i) {
         args[i].view = ctx->d_bviews.p + i;
-        args[i].out = raster_out(ctx, *frames[i], &views[i].out, args[i].mask_pitch);
+        args[i].out = raster_out(ctx, *frames[i], &views[i].out, args[i]);
         k.ptrs.insert(k.ptrs.end(), {views[i].scene, args[i].out.rgba8, args[i].out.rgb, args[i].out.final_t,
                                      args[i].out.n_contrib});
         k.dims.insert(k.dims.end(), {args[i].n, args[i].w, args[i].h});
@@ -1064,7 +1067,7 @@ static int enqueue_raster_backward(gs_ctx* ctx, Frame& f, const gs_scene* scene,
     f.grad2d_zero = false;
     if (ev) cudaEventRecord(ev[0], s);
     launch_raster_backward(ctx->cfg.tile_size, f.order.p, f.vals[f.sorted_buf].p, f.rec.p, scene->n, f.width,
-                           f.height, f.tiles_x, f.tiles_y, f.final_t.p, f.n_contrib.p, f.hit_masks.p, f.mask_pitch, dl,
+                           f.height, f.tiles_x, f.tiles_y, f.final_t.p, f.n_contrib.p, f.hit_masks(), f.mask_pitch, dl,
                            f.grad2d.p, s);
     if (ev) cudaEventRecord(ev[1], s);
     GS_CK(cudaGetLastError());
