@@ -373,7 +373,7 @@ void enqueue_views(gs_ctx* ctx, Frame* const* frames, const FrameArgs* args, uin
         emit[v] = EmitView{f.counts.p, f.meta.p, f.offsets.p, f.keys[0].p, f.vals[0].p, f.ctl.p, f.flags.p,
                            a.n, a.tiles_x, a.max_instance, a.passes};
         order[v] = OrderView{f.ranges.p, f.order_hist.p, f.order.p, f.ctl.p, tiles};
-        raster[v] = RasterView{f.order.p, f.vals[sorted].p, f.rec.p, a.out, a.n, a.w, a.h, a.tiles_x, tiles};
+        raster[v] = RasterView{f.order.p, f.vals[sorted].p, f.rec.p, a.out, &f.ctl.p->status, a.n, a.w, a.h, a.tiles_x, tiles};
         passes = std::max(passes, a.passes);
         key_bits = std::max(key_bits, 16u + bitlen(tiles - 1u));
     }

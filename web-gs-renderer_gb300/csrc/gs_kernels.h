@@ -199,6 +199,7 @@ struct RasterView {
     const uint32_t* vals;
     const float4* rec;
     RasterOut out;
+    uint32_t* status;  // the frame's status word (checked builds)
     uint32_t n, width, height, tiles_x, tiles;
 };
 void launch_raster(const RasterView* views, uint32_t count, uint32_t tile, uint32_t batch, cudaStream_t s);

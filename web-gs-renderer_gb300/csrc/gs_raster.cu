@@ -270,8 +270,10 @@ __device__ __forceinline__ void raster_view(const RasterView& view, uint32_t blo
         if (over) continue;
         const uint32_t groups = (cnt + 31u) / 32u;
         const uint32_t words = lane < groups ? cta.masks[lane][warp] : 0u;
-        if (LAST && lane < groups && out.hit_masks)  // the backward visits the same splats
-            out.hit_masks[plane * out.mask_pitch + hit_mask_base(start, tile) + ((i - start) >> 5) + lane] = words;
+        if (LAST && lane < groups && out.hit_masks) {  // the backward visits the same splats
+            const size_t at = hit_mask_base(start, tile) + ((i - start) >> 5) + lane;
+            if (GS_IN_BOUNDS(at, out.mask_pitch, view.status)) out.hit_masks[plane * out.mask_pitch + at] = words;
+        }
         uint32_t any = __ballot_sync(0xffffffffu, words != 0u);
         while (!over && (any != 0u || head < tail)) {
             if (any != 0u && tail - head < kChunk) {
