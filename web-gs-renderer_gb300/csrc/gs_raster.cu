@@ -185,7 +185,7 @@ __device__ __forceinline__ void raster_view(const RasterView& view, uint32_t blo
     float T = inside ? 1.0f : 0.0f, final_t = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
     uint32_t last = 0;
     uint32_t head = 0, tail = 0;             // hits blended, listed
-    bool over = false;                       // every pixel of the warp is done
+    bool over = __all_sync(0xffffffffu, T == 0.0f);  // every pixel of the warp is done, or none is in the image
 
     // blends the next cnt (at most kChunk) listed hits of the step whose first position is pos0
     auto blend = [&](uint32_t cnt, uint32_t pos0) {
