@@ -820,8 +820,8 @@ void launch_scan_emit(const EmitView* views, uint32_t count, uint32_t together, 
     const uint64_t all = (uint64_t)n * together;
     if (all < 75000u) launch(k_scan_emit<1>, k_scan_emit_views<1>, 1u);
     else if (all < 150000u) launch(k_scan_emit<2>, k_scan_emit_views<2>, 2u);
-    else if (n < 8000000u) launch(k_scan_emit<4>, k_scan_emit_views<4>, 4u);
-    else launch(k_scan_emit<8>, k_scan_emit_views<8>, 8u);
+    else if (n < 8000000u || count > 1) launch(k_scan_emit<4>, k_scan_emit_views<4>, 4u);
+    else launch_pdl(k_scan_emit<8>, dim3(n / kScanPartition + 1u), dim3(kScanThreads), s, views[0], digit_bits, slot);
 }
 
 void launch_exclusive_scan(uint32_t* data, uint32_t n, uint32_t* total_dev, FrameCtl* ctl, uint64_t* flags,
