@@ -1295,7 +1295,10 @@ int gs_autotune_scenes(const gs_config* base, const float* const* packed, const 
     std::vector<std::pair<float, gs_config>> timed;
     for (uint32_t t : tiles)
         for (uint32_t d : digits)
-            for (uint32_t r : batches)
+            for (uint32_t r : batches) {
+                // of depths that come to the same step (128 and 256, all of them in 8x8 tiles) the largest stands
+                // for them: 28 configurations, and the three that are timed again are three different ones
+                if (r < 256u && raster_step(t, r) == raster_step(t, 2u * r)) continue;
                 for (uint32_t sb : blocks) {
                     gs_config c = b;
                     c.tile_size = t;
@@ -1308,6 +1311,7 @@ int gs_autotune_scenes(const gs_config* base, const float* const* packed, const 
                     if (rc != GS_OK) return rc;
                     timed.emplace_back(ms, c);
                 }
+            }
     std::sort(timed.begin(), timed.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
     float best_t = 3.0e38f;
     gs_config best_c = b;

@@ -192,7 +192,8 @@ struct RasterOut {
 // leaves every tile ceil(length / 32) words of its own; a plane holds max_instance / 32 + tiles + 1.
 __host__ __device__ __forceinline__ size_t hit_mask_base(uint32_t start, uint32_t tile) { return (size_t)(start >> 5) + tile; }
 // configure_raster_kernels: kernel attributes, once per device. batch: a quarter of the range
-// positions staged per step (32 to 256; a step is 512 at most, 128 in 8x8 tiles). order: launch_tile_order's; n bounds the Gaussian indices.
+// positions staged per step (32 to 256; a step is 512 at most, 128 in 8x8 tiles: raster_step). order:
+// launch_tile_order's; n bounds the Gaussian indices.
 void configure_raster_kernels();
 struct RasterView {
     const uint4* order;
@@ -202,6 +203,7 @@ struct RasterView {
     uint32_t* status;  // the frame's status word (checked builds)
     uint32_t n, width, height, tiles_x, tiles;
 };
+uint32_t raster_step(uint32_t tile, uint32_t batch);
 void launch_raster(const RasterView* views, uint32_t count, uint32_t tile, uint32_t batch, cudaStream_t s);
 
 // y = the pinned exp of x (raster: the raster's exp, defined on [-5.6, 0]).

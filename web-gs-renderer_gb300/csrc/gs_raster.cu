@@ -310,7 +310,6 @@ k_raster_views(const __grid_constant__ Views<RasterView> views, uint32_t step) {
 template <int TILE>
 void launch_tile(const RasterView* views, uint32_t count, uint32_t step, cudaStream_t s) {
     constexpr uint32_t kSubs = TILE / RasterShared<TILE>::kSub;
-    step = std::min(step, RasterShared<TILE>::kStage);
     uint32_t tiles = 0;
     bool last = false, final_t = false;
     for (uint32_t v = 0; v < count; ++v) {
@@ -351,11 +350,16 @@ void configure_raster_kernels() {
     configure_tile<32>();
 }
 
+// positions per step (a multiple of 32), as far as the stage goes: most tiles need one or two
+uint32_t raster_step(uint32_t tile, uint32_t batch) {
+    return std::min(4u * batch, tile == 8 ? RasterShared<8>::kStage : RasterShared<16>::kStage);
+}
+
 void launch_raster(const RasterView* views, uint32_t count, uint32_t tile, uint32_t batch, cudaStream_t s) {
-    batch *= 4u;  // positions per step (a multiple of 32), as far as the stage goes: most tiles need one or two
-    if (tile == 8) launch_tile<8>(views, count, batch, s);
-    else if (tile == 32) launch_tile<32>(views, count, batch, s);
-    else launch_tile<16>(views, count, batch, s);
+    const uint32_t step = raster_step(tile, batch);
+    if (tile == 8) launch_tile<8>(views, count, step, s);
+    else if (tile == 32) launch_tile<32>(views, count, step, s);
+    else launch_tile<16>(views, count, step, s);
 }
 
 }  // namespace gs
