@@ -121,16 +121,19 @@ def algorithmic_bytes(fi: dict, n: int, pixels: int, passes: int) -> dict:
         # the tile ranges cleared, the control block's counters and digit histograms reset
         "frame begin": 8 * tiles + 8 * 1024,
         # 12 B position of every Gaussian + the other 224 B of each one in front of the near plane;
-        # writes: 4 B count each, 64 B raster record per near-plane survivor, 16 B rect per visible
-        "preprocess": 12 * n + 224 * npass + 4 * n + 64 * npass + 16 * vis,
+        # writes: 4 B count each, 48 B of the raster record per near-plane survivor, its 16 B of cull
+        # extents and the 16 B rect per visible
+        "preprocess": 12 * n + 224 * npass + 4 * n + 48 * npass + 32 * vis,
         # counts + rects in, offsets + keys/values out
         "scan+emit": 4 * (n + 1) + 16 * vis + 4 * (n + 1) + 8 * s,
         # each pass reads and writes keys and values (the last one also leaves the tile ranges)
         "sort": passes * 16 * s,
         # the ranges read twice (bin counts, placement), the order written with them
         "tile order": 2 * 8 * tiles + 16 * tiles,
-        # per instance the index and the 64 B record, per tile its place and range, per pixel 4 B rgba8
-        "raster": 68 * s + 16 * tiles + 4 * pixels,
+        # per instance the index, the centre and the cull extents (the record's other 40 B are read only
+        # for splats that meet a block, whose number no counter gives: a lower bound), per tile its
+        # place and range, per pixel 4 B rgba8
+        "raster": 28 * s + 16 * tiles + 4 * pixels,
     }
 
 
