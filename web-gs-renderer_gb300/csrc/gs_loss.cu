@@ -3,7 +3,7 @@
 // Gaussian window (sigma 1.5, normalised, separable), zero padding, C1 = 0.01^2, C2 = 0.03^2. With
 // the filtered moments m1 = G*x, m2 = G*x^2, mxy = G*(xy) the gradient is
 //   dSSIM/dx = G*(dS/dm1) + 2x G*(dS/dm2) + y G*(dS/dmxy)
-// (the window is symmetric). Two kernels, each on 32x16 output tiles of one channel with a 5-pixel
+// (the window is symmetric). Two kernels, each on 32x32 output tiles of one channel with a 5-pixel
 // halo staged in shared memory (both separable passes happen there):
 //   k_ssim_fwd  moments -> SSIM map -> its three partials (to global) + per-block SSIM and L1 sums;
 //   k_ssim_bwd  blurred partials + the L1 term -> dL/dx.

@@ -26,7 +26,7 @@
 // returns 512 bytes to a warp, four cycles of the SM's 128 bytes), 53% of the time at 1M / 1080p, the fp32
 // pipe 56%, issue 72%; where they are short (a dozen splats a tile at 1080p) the chain of loads, tile, index,
 // record, that each CTA goes through. So the tile comes with its range (k_tile_place), a record is read once
-// per tile, and 40 warps fit an SM (46 to 48 registers, 34 KB per CTA; 48 of them at 8x8 tiles). With 32 / 40 / 48
+// per tile, and 40 warps fit an SM (48 registers, 34 KB per CTA; 48 of them at 8x8 tiles, whose 40 registers spill 16 to 20 bytes). With 32 / 40 / 48
 // warps: 1M / 1080p 306 / 299 / 310 us a frame, 12 views of 300k in 32x32 tiles 745 / 710 / 738, 16 sparse
 // views of 35k at 1080p 370 / 339 / 340; steps of 256 cost 1M / 1080p 2%, of 768 gain nothing.
 //
