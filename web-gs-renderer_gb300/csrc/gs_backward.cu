@@ -78,17 +78,39 @@ __device__ __forceinline__ void pix_load(PixState& p, uint32_t x, uint32_t y, ui
     }
 }
 
-// Visits two splats for one pixel, the one at the higher position first (back to front): the same power / exp /
-// alpha decisions as the forward (bit for bit); gp = dL/dpower and the blending weight w of each, zeros where the
-// pixel did not blend it. T is recovered by division (the approximate reciprocal, 1 ulp, of 1 - alpha >= 0.01 is
+// Visits the splat at 1-based range position pos for one pixel: the same power / exp / alpha
+// decisions as the forward (bit for bit); gp = dL/dpower and its blending weight w, zeros if the pixel
+// did not blend it. T is recovered by division (the approximate reciprocal, 1 ulp, of 1 - alpha >= 0.01 is
 // accurate enough for a gradient). With C = sum_i alpha_i T_i c_i and T_{i+1} = T_i (1 - alpha_i),
 // dC/dalpha_i = T_i c_i - S_i / (1 - alpha_i), S_i being the colour added behind splat i, so
 // dL/dalpha_i = T_i K_i - D_i / (1 - alpha_i) with K_i = dC . c_i and D_i = dC . S_i, and D grows by
 // alpha_i T_i K_i per step. No branch on the rejections: a rejected pixel takes alpha = 0 and K = 0, which
-// leaves its state as it is, and gives two zeros, also where D is no longer finite. What does not depend on the
-// pixel's state is formed for both splats at once by packed operations (each half rounds like the scalar form).
+// leaves its state as it is, and gives two zeros, also where D is no longer finite.
+__device__ __forceinline__ void pix_step(PixState& p, uint32_t pos, const float4& a, const float4& b,
+                                         const float2& c, float& gp, float& w) {
+    const float dx = a.x - p.fx, dy = a.y - p.fy;
+    const float power = __fmaf_rn(-0.5f, __fmaf_rn(a.z * dx, dx, (b.x * dy) * dy), -((a.w * dx) * dy));
+    // the forward's o * exp(power); a positive cut-off: the opacity itself is below 1/255
+    const float og = raster_alpha_unclamped(c.y > 0.0f ? 0.0f : b.y, max_nan(power, kPowerFloor));
+    float alpha = fminf(kAlphaClamp, og);
+    // from here on only gradients are formed: fused multiply-adds are fine (the decisions
+    // follow the forward's pinned arithmetic)
+    float k = __fmaf_rn(b.z, p.dr, __fmaf_rn(b.w, p.dg, c.x * p.db));  // dC . c
+    const bool in = (pos <= p.L) & !(power > 0.0f) & (alpha >= kEpsilon);
+    alpha = in ? alpha : 0.0f;
+    k = in ? k : 0.0f;
+    const float ria = fast_rcp(1.0f - alpha);
+    p.T = p.T * ria;  // transmittance in front of this splat
+    w = alpha * p.T;
+    const float dalpha = __fmaf_rn(p.T, k, -(p.d * ria));
+    gp = in & (og <= kAlphaClamp) ? dalpha * alpha : 0.0f;  // a clamped alpha passes no gradient
+    p.d = __fmaf_rn(w, k, p.d);
+}
+
+// The same for two splats, the one at the higher position first (back to front): what does not depend on the
+// pixel's state is formed for both at once by packed operations (each half rounds like the scalar form).
 // Pairs as the walk lays them out; opacity 0 stands for one below every cut-off (its alpha is 0).
-__device__ __forceinline__ void pix_step(PixState& p, const float4& p0, const float4& p1, const float4& p2,
+__device__ __forceinline__ void pix_step2(PixState& p, const float4& p0, const float4& p1, const float4& p2,
                                           const float4& p3, const float4& p4, float2& gp, float2& w) {
     const float2 dx = __fadd2_rn(make_float2(p0.x, p0.y), both(-p.fx)), dy = __fadd2_rn(make_float2(p0.z, p0.w), both(-p.fy));
     const float2 q = __ffma2_rn(__fmul2_rn(make_float2(p1.x, p1.y), dx), dx,
@@ -112,6 +134,63 @@ __device__ __forceinline__ void pix_step(PixState& p, const float4& p0, const fl
     };
     one(power.x, og.x, kk.x, __float_as_uint(p4.z), gp.x, w.x);
     one(power.y, og.y, kk.y, __float_as_uint(p4.w), gp.y, w.y);
+}
+
+__device__ __forceinline__ bool pix_finite(const PixState& p) {
+    return finite_f(p.dr) && finite_f(p.dg) && finite_f(p.db);
+}
+
+// The walk of a block with a pixel whose dL/dC is not finite. Such a pixel must not reach the splats that it does
+// not blend, where zero times it would be NaN, so the sums over the block take the pixels that blend a splat one
+// by one (selects, nine shuffle sums per hit) instead of the flush's plain products. Its own function, so that the
+// common walk spends nothing on it: the choice within the flush cost 3% at 1M / 1080p (260 -> 267 us) and 8% at
+// 20k / 397x301. Step of an image of NaN at 1M / 1080p 1.04 ms (a finite one 0.33), with one
+// such pixel in 1000 0.365; 4.9 and 0.71 when each of them walked its tile's list by itself.
+__device__ __noinline__ void walk_not_finite(PixState p, uint32_t wmax, const uint32_t* __restrict__ masks,
+                                             const uint32_t* __restrict__ vals, const float4* __restrict__ rec,
+                                             uint32_t n, float* __restrict__ grad2d) {
+    constexpr uint32_t kAll = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t group = (wmax + 31u) >> 5; group-- > 0u;) {
+        uint32_t m = masks[group];
+        const uint32_t last = wmax - (group << 5);  // positions of the group that are visited
+        if (last < 32u) m &= (1u << last) - 1u;
+        if (m == 0u) continue;
+        // a lane holds one of the group's splats
+        const uint32_t mine = m >> lane & 1u ? vals[(group << 5) + lane] : n;
+        float4 ra = make_float4(0.0f, 0.0f, 0.0f, 0.0f), rb = ra, rc = ra;
+        if (mine < n) {
+            ra = rec[(size_t)kRecFloat4 * mine];
+            rb = rec[(size_t)kRecFloat4 * mine + 1];
+            rc = rec[(size_t)kRecFloat4 * mine + 2];
+        }
+        while (m != 0u) {
+            const int bit = 31 - __clz(m);
+            m &= ~(1u << bit);
+            const uint32_t gi = __shfl_sync(kAll, mine, bit);
+            if (gi >= n) continue;  // only after a timed-out sort
+            auto from = [&](float v) { return __shfl_sync(kAll, v, bit); };
+            const float4 a = make_float4(from(ra.x), from(ra.y), from(ra.z), from(ra.w));
+            const float4 b = make_float4(from(rb.x), from(rb.y), from(rb.z), from(rb.w));
+            const float2 c = make_float2(from(rc.x), from(rc.y));
+            float gp, w;
+            pix_step(p, (group << 5) + (uint32_t)bit + 1u, a, b, c, gp, w);
+            const bool on = w != 0.0f;  // blended (a blended pair's weight is positive)
+            if (!__any_sync(kAll, on)) continue;
+            const float dx = a.x - p.fx, dy = a.y - p.fy, gx = gp * dx, gy = gp * dy;
+            float v[9] = {gp, gx, gy, gx * dx, gx * dy, gy * dy, w * p.dr, w * p.dg, w * p.db};
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                v[k] = on ? v[k] : 0.0f;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(kAll, v[k], o);
+            }
+            float* q = grad2d + (size_t)8 * gi;
+            red_add4_if(lane == 0u, q, -__fmaf_rn(a.z, v[1], a.w * v[2]), -__fmaf_rn(b.x, v[2], a.w * v[1]), v[6], v[7]);
+            red_add4_if(lane == 1u, q + 4, -0.5f * v[3], -v[4], -0.5f * v[5], v[8]);
+            red_add_if(lane == 2u, grad2d + (size_t)8 * n + gi, v[0] / b.y);
+        }
+    }
 }
 
 constexpr uint32_t kRowPitch = 36;  // floats per row: 32 pixels, padded so that the eight lanes that read
@@ -174,7 +253,11 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
     pix_load(p, bx0 + (lane & 7u), by0 + (lane >> 3), width, height, final_t, n_contrib, dl_drgb);
     const uint32_t wmax = min(__reduce_max_sync(0xffffffffu, p.L), len);
     if (wmax == 0u) return;
-    const bool all_finite = __all_sync(0xffffffffu, finite_f(p.dr) && finite_f(p.dg) && finite_f(p.db));
+    const uint32_t* const masks = hit_masks + (size_t)warp * mask_pitch + hit_mask_base(start, tile);
+    if (!__all_sync(0xffffffffu, pix_finite(p))) {
+        walk_not_finite(p, wmax, masks, vals + start, rec, n, grad2d);
+        return;
+    }
     // of a flush a lane sums hit fr over row fc of the block: the row's dL/dC, in pairs of pixels
     const uint32_t fr = lane >> 2, fc = lane & 3u;
     float2 dr[4], dg[4], db[4];
@@ -217,7 +300,7 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
         for (uint32_t u = 0; u < kHits / 2u; ++u) {
             const float4* r = sh.pair[4u * v + u];
             float2 gp, w;
-            pix_step(p, r[0], r[1], r[2], r[3], r[4], gp, w);
+            pix_step2(p, r[0], r[1], r[2], r[3], r[4], gp, w);
             sh.gp[2u * u][lane] = gp.x;
             sh.gp[2u * u + 1u][lane] = gp.y;
             sh.w[2u * u][lane] = w.x;
@@ -237,6 +320,7 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
         const float x0 = a.x - row_x, dy = a.y - row_y;
         float2 dx = make_float2(x0, x0 - 1.0f);
         float2 t = __fmul2_rn(g[0], dx), s0 = g[0], sx = t, sxx = __fmul2_rn(t, dx);
+        float2 r = __fmul2_rn(wt[0], dr[0]), gr = __fmul2_rn(wt[0], dg[0]), bl = __fmul2_rn(wt[0], db[0]);
 #pragma unroll
         for (uint32_t k = 1; k < 4u; ++k) {
             dx = __fadd2_rn(dx, both(-2.0f));
@@ -244,32 +328,15 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
             s0 = __fadd2_rn(s0, g[k]);
             sx = __fadd2_rn(sx, t);
             sxx = __ffma2_rn(t, dx, sxx);
+            r = __ffma2_rn(wt[k], dr[k], r);
+            gr = __ffma2_rn(wt[k], dg[k], gr);
+            bl = __ffma2_rn(wt[k], db[k], bl);
         }
-        auto weighted = [&](const float2 (&d)[4]) {
-            float2 v = __fmul2_rn(wt[0], d[0]);
-#pragma unroll
-            for (uint32_t k = 1; k < 4u; ++k) v = __ffma2_rn(wt[k], d[k], v);
-            return v.x + v.y;
-        };
-        // a pixel whose dL/dC is not finite must not reach the splats that it does not blend: zero times it
-        // would be NaN (a blended pair's weight is positive). A whole image of NaN at 1M / 1080p takes 0.376 ms
-        // (a finite one 0.338, and 4.9 where such pixels walked their tile's list one by one).
-        auto weighted_blended = [&](const float2 (&d)[4]) {
-            float v = 0.0f;
-#pragma unroll
-            for (uint32_t k = 0; k < 4u; ++k) {
-                v += wt[k].x != 0.0f ? wt[k].x * d[k].x : 0.0f;
-                v += wt[k].y != 0.0f ? wt[k].y * d[k].y : 0.0f;
-            }
-            return v;
-        };
-        const float red = all_finite ? weighted(dr) : weighted_blended(dr), green = all_finite ? weighted(dg) : weighted_blended(dg);
-        const float blue = all_finite ? weighted(db) : weighted_blended(db);
         // sums over the row: gp, gp dx, gp dy, gp dx^2, gp dx dy, gp dy^2, w dC
         float sum0 = s0.x + s0.y;
         const float rx = sx.x + sx.y, ry = dy * sum0;
-        const float even[4] = {rx, ry, red, green};
-        const float odd[4] = {sxx.x + sxx.y, dy * rx, dy * ry, blue};
+        const float even[4] = {rx, ry, r.x + r.y, gr.x + gr.y};
+        const float odd[4] = {sxx.x + sxx.y, dy * rx, dy * ry, bl.x + bl.y};
         // and over the four rows: the even lanes of a hit get the first four, the odd ones the others
         const bool first = (fc & 1u) == 0u;
         float v4[4];
@@ -294,7 +361,6 @@ __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backw
 
     // the groups of 32 positions with hits, from the top down: masks are read 32 groups at a time, and the
     // Gaussian indices of a group are loaded while the group before it is staged
-    const uint32_t* const masks = hit_masks + (size_t)warp * mask_pitch + hit_mask_base(start, tile);
     int32_t group = (int32_t)((wmax - 1u) >> 5) + 1;  // the group staged last
     uint32_t words = 0, left = 0;   // the lane's mask word of the current 32 groups; how many are unread
     uint32_t m = 0, gnext = n;      // the next group's mask and this lane's Gaussian in it
