@@ -185,7 +185,9 @@ __device__ __forceinline__ void raster_view(const RasterView& view, uint32_t blo
     float T = inside ? 1.0f : 0.0f, final_t = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
     uint32_t last = 0;
     uint32_t head = 0, tail = 0;             // hits blended, listed
-    bool over = __all_sync(0xffffffffu, T == 0.0f);  // every pixel of the warp is done, or none is in the image
+    // every pixel of the warp is done, or none is in the image. The same question in two forms: 16x16 tiles with the
+    // second lose 0.4% of a frame (1M / 1080p 335.2 -> 336.4 us), 32x32 ones with the first 1.1% (16 views 2433 -> 2460)
+    bool over = TILE < 32 ? __all_sync(0xffffffffu, !inside) : __all_sync(0xffffffffu, T == 0.0f);
 
     // blends the next cnt (at most kChunk) listed hits of the step whose first position is pos0
     auto blend = [&](uint32_t cnt, uint32_t pos0) {
