@@ -139,17 +139,17 @@ def algorithmic_bytes(fi: dict, n: int, pixels: int, passes: int) -> dict:
 
 # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum, one ncu --set full capture of
 # the forward frame of this workload on a GB300) and what bounds each kernel there.
-NCU_TRAFFIC_BYTES = {"preprocess": 307.8e6, "raster": 61.0e6}
+NCU_TRAFFIC_BYTES = {"preprocess": 307.8e6, "raster": 61.1e6}
 # issue-slot utilisation of the kernels bound by instruction issue (ncu smsp__issue_active, one
 # capture of the kernel at this workload): for them this, not the HBM fraction, is the efficiency measure
-NCU_ISSUE_ACTIVE = {"raster": 0.737}
+NCU_ISSUE_ACTIVE = {"raster": 0.736}
 # warp instructions per launch (ncu smsp__inst_executed.sum, the same capture): the numerator of the
 # issue-rate roofline of those kernels (four issue slots per SM per cycle)
-NCU_WARP_INSTRUCTIONS = {"raster": 180.27e6}
+NCU_WARP_INSTRUCTIONS = {"raster": 179.89e6}
 LIMITER = {
-    "raster": "instruction issue, the fp32 pipe and shared-memory reads together (ncu: issue slots busy 73.7%, "
-              "fp32 pipe 59%, shared-memory data 55%, DRAM 4% of peak; the 64-byte records are re-read from L2, so "
-              "DRAM traffic is below the algorithmic bytes)",
+    "raster": "instruction issue, the fp32 pipe and shared-memory reads together (ncu: issue slots busy 73.6%, "
+              "fp32 pipe 59%, shared-memory data 55%, DRAM 4% of peak; the records are re-read from L2 per tile, so "
+              "DRAM traffic is below the bytes charged)",
     "preprocess": "HBM and the pinned arithmetic (ncu: 70% of issue slots)",
 }
 

@@ -217,10 +217,11 @@ struct BwdWarp {
 // batches, computed the cull again and met at two barriers per batch, a hit's bookkeeping (finding the
 // next bit, addresses, the counter of the pending rows) is gone.
 //
-// Bound by instruction issue and shared-memory reads where the blocks fill the GPU, by the longest list otherwise. Measured against a CTA per tile with shuffle
-// reductions and two pixels per lane, mixture scenes: 1M / 1080p 405 -> 260 us; 500k / 720p (a list of 2300 splats)
-// 358 -> 129; 20k / 397x301 92 -> 24. On the way, with the block's sums on matrix instructions (above), 1M /
-// 1080p in thousand cycles, from 839: the chain's divide as one reciprocal and no branch in a hit 693 -> 664;
+// Bound by instruction issue (76% of slots at 29 warps per SM) and shared-memory reads (74%) where the
+// blocks fill the GPU, by the longest list otherwise. Measured against a CTA per tile with shuffle
+// reductions and two pixels per lane, mixture scenes: 1M / 1080p 405 -> 260 us; 3M / 1080p (mean of
+// eight views) 879 -> 526; 500k / 720p (a list of 2300 splats) 358 -> 130; 20k / 397x301 92 -> 23.4. On the
+// way, with the block's sums on matrix instructions (above), 1M / 1080p in thousand cycles, from 839: the chain's divide as one reciprocal and no branch in a hit 693 -> 664;
 // predicated atomics 631; hits in pairs on packed operations 577, their loop fully unrolled 560.
 template <int TILE>
 __global__ void __launch_bounds__(kBwdWarps * 32, 32 / kBwdWarps) k_raster_backward(const uint4* __restrict__ order,

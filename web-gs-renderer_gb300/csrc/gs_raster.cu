@@ -26,14 +26,15 @@
 // returns 512 bytes to a warp, four cycles of the SM's 128 bytes), 53% of the time at 1M / 1080p, the fp32
 // pipe 56%, issue 72%; where they are short (a dozen splats a tile at 1080p) the chain of loads, tile, index,
 // record, that each CTA goes through. So the tile comes with its range (k_tile_place), a record is read once
-// per tile, and 40 warps fit an SM (48 registers, 34 KB per CTA; 48 of them at 8x8 tiles, whose 40 registers spill 16 to 20 bytes). With 32 / 40 / 48
-// warps: 1M / 1080p 306 / 299 / 310 us a frame, 12 views of 300k in 32x32 tiles 745 / 710 / 738, 16 sparse
-// views of 35k at 1080p 370 / 339 / 340; steps of 256 cost 1M / 1080p 2%, of 768 gain nothing.
+// per tile, and 40 warps fit an SM (46 to 48 registers, of which the plain 16x16 frame spills one; 34 KB per
+// CTA; 48 warps at 8x8 tiles, whose 40 registers spill 16 to 20 bytes). With 32 / 40 / 48 warps: 1M / 1080p
+// 306 / 299 / 310 us a frame, 12 views of 300k in 32x32 tiles 745 / 710 / 738, 16 sparse views of 35k at 1080p
+// 370 / 339 / 340; steps of 256 cost 1M / 1080p 2%, of 768 gain nothing.
 //
 // Measured against one CTA per tile that staged 256 splats between two barriers, computed the octagon per
 // tile and splat and walked the bits of its ballots at one splat per step (32 registers, 2048 threads per
 // SM): 1M / 1080p 189.5 -> 162.4 us (216M -> 143M warp instructions), 3M / 4K 1168 -> 930, 250k / 1237x823 in
-// 8x8 tiles 105 -> 70, a close-up of 60k at 1600x900 212 -> 177, 16 views in 32x32 tiles 3906 -> 2198 in
+// 8x8 tiles 105 -> 70, a close-up of 60k at 1600x900 212 -> 176, 16 views in 32x32 tiles 3906 -> 2167 in
 // sum, 50k / 512x512 47.6 -> 41.7, the sixteen sparse views 341 -> 344. Other ways to bring the records
 // in: all of a step's, hit or not, 178.3, 1024, 75.3, 182, 2495, 42.7 and 346 us (a list takes its splats by their
 // bounding squares, so many of them meet no block); a ring of hits per warp, filled while the hits
