@@ -39,7 +39,7 @@ template <class T> struct DevBuf {
 #ifdef GS_CHECKED
         const size_t bytes = want * sizeof(T);
         cudaError_t e = cudaMalloc(&raw, bytes + 2 * kCanaryBytes);
-        if (e != cudaSuccess) { raw = nullptr; return e; }
+        if (e != cudaSuccess) { cudaGetLastError(); raw = nullptr; return e; }  // not left for the next call to find
         e = cudaMemset(raw, 0xA5, kCanaryBytes);
         if (e == cudaSuccess) e = cudaMemset(raw + kCanaryBytes + bytes, 0xA5, kCanaryBytes);
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -47,7 +47,7 @@ template <class T> struct DevBuf {
         p = reinterpret_cast<T*>(raw + kCanaryBytes);
 #else
         cudaError_t e = cudaMalloc(&p, want * sizeof(T));
-        if (e != cudaSuccess) { p = nullptr; return e; }
+        if (e != cudaSuccess) { cudaGetLastError(); p = nullptr; return e; }  // not left for the next call to find
 #endif
         cap = want;
         return cudaSuccess;
@@ -278,9 +278,12 @@ int frame_args(gs_ctx* ctx, const gs_scene* scene, const gs_view* view, FrameArg
     return GS_OK;
 }
 
-// Grows a frame's buffers for the frame described by a.
+// Grows a frame's buffers for the frame described by a. The last frame is gone with the first buffer that is
+// replaced, also if a later one fails.
 int ensure_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a) {
     const uint32_t radix = 1u << ctx->cfg.digit_bits;
+    const bool valid = f.valid;
+    f.valid = false;
     const void* before[] = {f.rec.p, f.meta.p, f.counts.p, f.offsets.p, f.keys[0].p, f.keys[1].p, f.vals[0].p,
                             f.vals[1].p, f.flags.p, f.ranges.p, f.rgba8.p, f.rgb.p, f.final_t.p, f.n_contrib.p,
                             f.order.p, f.order_hist.p};
@@ -312,6 +315,7 @@ int ensure_frame(gs_ctx* ctx, Frame& f, const FrameArgs& a) {
                            f.vals[1].p, f.flags.p, f.ranges.p, f.rgba8.p, f.rgb.p, f.final_t.p, f.n_contrib.p,
                            f.order.p, f.order_hist.p};
     if (std::memcmp(before, after, sizeof(before)) != 0) ++ctx->alloc_gen;
+    else f.valid = valid;
     return GS_OK;
 }
 
